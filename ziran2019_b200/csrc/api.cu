@@ -475,7 +475,7 @@ int zmpm_destroy(zmpm_ctx* ctx)
         &ctx->group_page, &ctx->group_nbr, &ctx->emit_flag, &ctx->emit_scan, &ctx->page_first, &ctx->page_block, &ctx->block_page,
         &ctx->block_index, &ctx->gm, &ctx->gmv, &ctx->vn, &ctx->dv, &ctx->vstar, &ctx->facc, &ctx->res, &ctx->proj, &ctx->collided,
         &ctx->node_idx, &ctx->red, &ctx->scal, &ctx->counters, &ctx->dcolliders, &ctx->adm_F, &ctx->adm_gvn, &ctx->adm_B, &ctx->adm_pre,
-        &ctx->adm_rhs, &ctx->adm_w, &ctx->adj, &ctx->kvf, &ctx->vstarf, &ctx->pfn, &ctx->pfsc, &ctx->gsync };
+        &ctx->adm_rhs, &ctx->adm_w, &ctx->adm_K, &ctx->adm_nbr, &ctx->adj, &ctx->kvf, &ctx->vstarf, &ctx->pfn, &ctx->pfsc, &ctx->gsync };
     for (DBuf* b : bufs) b->release();
     for (auto& b : ctx->kv) b.release();
     for (auto* v : { &ctx->ckpt_pd, &ctx->ckpt_pi, &ctx->ckpt_sid })
@@ -1048,9 +1048,10 @@ static int substep_finish(zmpm_ctx* ctx, double dt, const zmpm_solver& s, zmpm_s
     st->svd_fp64_reevaluations = hc.svd_fp64;
     if (!admm && !expl) ctx->fp64_res_run = hs.fp64_res ? ctx->fp64_res_run + 1 : 0;
     // ADMM iteration: collision, local step, force scatter, operator, start,
-    // Krylov start, persistent MINRES, dv update, dual update, advance
+    // Krylov start, persistent MINRES, dv update, dual update, advance (the
+    // assembled operator: its product is part of the start)
     if (ctx->graph_used && admm)
-        g_kernel_launches += 10 * (int64_t)hs.nit;
+        g_kernel_launches += (ctx->admm_stencil ? 9 : 10) * (int64_t)hs.nit;
     else if (ctx->graph_used)
         g_kernel_launches += newton_body_launches(ctx) * (int64_t)hs.nit;
     ctx->graph_used = false;

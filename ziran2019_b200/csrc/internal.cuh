@@ -217,6 +217,8 @@ struct Ctx {
     // global-operator coefficients B [6][Pcap] (HVP precision); node
     // preconditioner, right-hand side and transfer weights
     DBuf adm_F, adm_gvn, adm_B, adm_pre, adm_rhs, adm_w;
+    DBuf adm_K, adm_nbr;                  // assembled global operator [B][125][NPB] (HVP precision) and the pages' neighbours (stencil.cu)
+    bool admm_stencil = false;            // the last ADMM substep ran on it (launch accounting)
     DBuf adj;                             // adjoint particle arrays [AJ_FIELDS][Pcap]
     std::vector<DBuf> ckpt_pd, ckpt_pi, ckpt_sid; // device checkpoints
     std::vector<double> ckpt_time;

@@ -21,23 +21,15 @@
 
 #include "hvp.cuh"
 #include "internal.cuh"
+#include "krylov.cuh"
 #include "mat3.cuh"
 #include "node.cuh"
+#include "stencil.cuh"
 
 namespace zmpm {
 
 int launch_p2g(Ctx* ctx);
 int launch_g2p(Ctx* ctx, bool plastic);
-
-__device__ __forceinline__ void project3(const int8_t* col, const double* P6, int64_t nn, int64_t n, double v[3])
-{
-    if (!col[n]) return;
-    double p00 = P6[n], p01 = P6[nn + n], p02 = P6[2 * nn + n], p11 = P6[3 * nn + n], p12 = P6[4 * nn + n], p22 = P6[5 * nn + n];
-    double a = v[0], b = v[1], c = v[2];
-    v[0] = p00 * a + p01 * b + p02 * c;
-    v[1] = p01 * a + p11 * b + p12 * c;
-    v[2] = p02 * a + p12 * b + p22 * c;
-}
 
 // ------------------------------------------------------- collision query --
 // AnalyticLevelSet::queryInside for half space, sphere and axis-aligned box.
@@ -364,33 +356,6 @@ __global__ void __launch_bounds__(ND_THREADS) k_residual(NodeGeom ng, const doub
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// Solver buffers of one linear solve.  MINRES rotates its three Lanczos
-// vectors Q, three search directions M and two preconditioned vectors Z by the
-// iteration index k read from device memory, so the same kernels (and the same
-// graph body) serve every iteration.
-struct KrylovBufs {
-    double *x, *r, *p, *q, *tmp;      // CG
-    double *Q[3], *M[3], *Z[2];       // MINRES
-    float* Zf[2];                     // FP32 node-major copies of Z ([B][NPB][4]) for the FP32 product (MIXED MINRES), or null
-    float* pf;                        // FP32 node-major copy of p for the FP32 product (MIXED CG), or null
-    double* hacc;                     // Hessian accumulator
-    const double* pre;                // diagonal preconditioner per node (the mass for Newton)
-};
-
-struct NewtonParams {
-    int32_t minres, kmax, nmax;
-    int32_t escalate;                 // MIXED: FP64 residual once the FP32 one stalls
-    double tol, abs_tol, tol_scale, dt;
-};
-
-__device__ __forceinline__ bool krylov_off(const SolverScalars* sc) { return sc->newton_done || !sc->kactive; }
-
-// Role selection by iteration index without indexing the parameter arrays at
-// run time (which would copy the kernel parameters to local memory).
-__device__ __forceinline__ double* sel3(double* const (&a)[3], int i) { return i == 0 ? a[0] : (i == 1 ? a[1] : a[2]); }
-template <class T>
-__device__ __forceinline__ T* sel2(T* const (&a)[2], int i) { return i == 0 ? a[0] : a[1]; }
-
 // The Newton residual of k_residual fused with the operands of the linear
 // solve's start, in one node pass: r = project(dt m g + dt f - m dv), facc
 // zeroed, x = 0, and from r the Krylov start vectors (CG: r, q = p = r/pre;
@@ -572,89 +537,6 @@ __global__ void __launch_bounds__(ND_THREADS) k_apply_A(NodeGeom ng, const doubl
     apply_A_body<NPB, false>(ng, gm, col, P6, dt2, xin, hacc, out, nullptr, 0);
 }
 
-// MINRES keeps its Lanczos vectors Q_j and preconditioned vectors Z_j
-// unnormalised (Minres.h:170-173 divides them by beta_j at the end of
-// iteration j - 1); every reader divides by beta_j, the same rounding as the
-// stored normalised vector.  beta_j = 0 leaves them as they are, as there.
-__device__ __forceinline__ double mr_norm(double v, double beta) { return beta > 0 ? v / beta : v; }
-
-// The search direction of iteration j = k - 1 (Minres.h:167-170):
-// M_j = (Z_j - delta M_{j-1} - epsilon M_{j-2}) / gamma, then x += t M_j.
-// The Lanczos step computes its scalars; the vector update runs in the next
-// iteration's operator pass or, after the last iteration, where the solve's x
-// is used (k_newton_step, k_admm_dv_update).
-struct MrPending {
-    const double *z, *m1, *m2;
-    double* out;
-    double delta, eps, gamma, t, beta;
-    bool on;
-};
-__device__ __forceinline__ MrPending mr_pending(const KrylovBufs& kb, const double* pend, int k)
-{
-    MrPending p;
-    p.on = k > 0;
-    p.z = sel2(kb.Z, (k + 1) & 1);   // Z_{k-1}, unnormalised
-    p.m1 = sel3(kb.M, (k + 1) % 3);  // M_{k-2}
-    p.m2 = sel3(kb.M, k % 3);        // M_{k-3}
-    p.out = sel3(kb.M, (k + 2) % 3); // M_{k-1}
-    p.delta = pend[0];
-    p.eps = pend[1];
-    p.gamma = pend[2];
-    p.t = pend[3];
-    p.beta = pend[4];                // beta_{k-1}
-    return p;
-}
-__device__ __forceinline__ double mr_direction(const MrPending& p, int64_t i)
-{
-    return (mr_norm(p.z[i], p.beta) - p.delta * p.m1[i] - p.eps * p.m2[i]) / p.gamma;
-}
-
-// The Givens update of MINRES iteration k (Minres.h:151-175): from the state
-// cur of iteration k (Minres.h:16-24), alpha = Z_k . W, beta_k and dz =
-// Z~_{k+1} . Q~_{k+1}, the state of iteration k + 1 into nx and the deferred
-// search direction's delta, epsilon, gamma, t and beta into pend; returns the
-// preconditioned residual norm.
-__device__ __forceinline__ double mr_givens(const double* cur, double alpha, double beta_k, double dz, double* nx, double* pend)
-{
-    const double beta_kp1 = sqrt(dz > 0 ? dz : 0.0);
-    // Gkm2 = Gkm1, Gkm1 = Gk
-    double c2 = cur[MR_GC1], s2 = cur[MR_GS1], c1 = cur[MR_GC0], s1 = cur[MR_GS0];
-    double e0 = c2 * 0 - s2 * beta_k, e1 = s2 * 0 + c2 * beta_k;
-    const double epsilon = e0;
-    double d0 = c1 * e1 - s1 * alpha, d1 = s1 * e1 + c1 * alpha;
-    const double delta = d0;
-    double t0 = d1, t1 = beta_kp1;
-    double c0 = 1, s0 = 0;
-    {
-        double dd = t0 * t0 + t1 * t1;
-        double sd = sqrt(dd);
-        if (sd != 0) {
-            double tt = 1 / sd;
-            c0 = t0 * tt;
-            s0 = -t1 * tt;
-        }
-    }
-    const double gamma = c0 * t0 - s0 * t1;
-    const double r0 = cur[MR_RHS0], r1 = cur[MR_RHS1];
-    const double tk = c0 * r0 - s0 * r1;
-    const double residual = s0 * r0 + c0 * r1;
-    nx[MR_GC0] = c0;
-    nx[MR_GS0] = s0;
-    nx[MR_GC1] = c1;
-    nx[MR_GS1] = s1;
-    nx[MR_GC2] = c2;
-    nx[MR_GS2] = s2;
-    nx[MR_RHS0] = residual;
-    nx[MR_RHS1] = 0;
-    nx[MR_BETA_KP1] = beta_kp1;
-    pend[0] = delta;
-    pend[1] = epsilon;
-    pend[2] = gamma;
-    pend[3] = tk;
-    pend[4] = beta_k;
-    return residual < 0 ? -residual : residual;
-}
-
 // ------------------------------------------------ persistent Krylov -----
 // One cooperative launch runs a whole linear solve of the Newton iteration
 // (ConjugateGradient::solve, ConjugateGradient.h:99-147, on the Newton
@@ -665,70 +547,6 @@ __device__ __forceinline__ double mr_givens(const double* cur, double alpha, dou
 // the same fixed order, so all hold bit-identical scalars and take the same
 // loop decision.  The barrier waits are bounded: a CTA that gives up raises
 // FLAG_TIMEOUT and the abort flag, and every CTA returns at its next barrier.
-
-// Block sum for FUSED_THREADS threads; the result in every thread.
-__device__ __forceinline__ double block_sum_fused(double v)
-{
-    __shared__ double ws[FUSED_THREADS / 32];
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) ws[w] = v;
-    __syncthreads();
-    double t = 0;
-#pragma unroll
-    for (int i = 0; i < FUSED_THREADS / 32; ++i) t += ws[i];
-    return t;
-}
-// Sum of n partials written by other CTAs of this kernel (read through L2), in
-// a fixed order identical in every CTA.
-__device__ __forceinline__ double reduce_partials_fused(const double* part, int n)
-{
-    double s = 0;
-    for (int i = threadIdx.x; i < n; i += FUSED_THREADS) s += __ldcg(part + i);
-    return block_sum_fused(s);
-}
-
-// Bounded grid-wide barrier (sense by generation count).  Returns false in
-// every thread of the CTA when this CTA gave up after `limit` polls or another
-// CTA did; the caller then returns.
-__device__ __forceinline__ bool grid_sync(GridSync* gs, long long limit, int32_t* flags)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned* vgen = &gs->gen;
-        volatile unsigned* vabort = &gs->abort;
-        int good = 1;
-        const unsigned g = *vgen;
-        __threadfence();
-        if (atomicAdd(&gs->count, 1u) == gridDim.x - 1) {
-            gs->count = 0;
-            __threadfence();
-            atomicAdd(&gs->gen, 1u);
-        }
-        else {
-            long long it = 0;
-            while (*vgen == g) {
-                if (*vabort) {
-                    good = 0;
-                    break;
-                }
-                if (++it > limit) {
-                    atomicOr(flags, (int32_t)FLAG_TIMEOUT);
-                    atomicExch(&gs->abort, 1u);
-                    good = 0;
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        if (*vabort) good = 0;
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-}
 
 struct HvpArgs {
     const int32_t *group_start, *group_nbr, *pi;
@@ -942,9 +760,6 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
 // from it).  Three bounded grid barriers per iteration: the product is
 // complete before the operator pass reads hacc, W before the Lanczos step, and
 // Z~_{k+1} before the next product and the reduction of its norm.
-// Nodes per thread and step in the node passes of k_mr_persistent (their
-// loads all issue before the arithmetic: the passes are latency-bound).
-constexpr int MR_UNROLL = 2;
 template <class L, class T, class TX, class Model>
 __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng, HvpArgs ha, Model model, const double* __restrict__ gm,
     const int8_t* __restrict__ col, const double* __restrict__ P6, double dt2, KrylovBufs kb, double* __restrict__ part_a,
@@ -954,16 +769,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng,
     constexpr int NPB = L::NPB;
     constexpr int CH = sizeof(T) == 4 ? 512 : 192;
     __shared__ HvpSmem<L, T, TX, CH> hs;
-    // the MINRES state of iteration k (Minres.h:16-24), then the deferred
-    // direction's scalars, beta_{k-1} and the residual norm
-    __shared__ double mst[12 + 5 + 2];
-    double* const pend = mst + 12;
+    __shared__ double mst[MST_N];
+    double* const pend = mst + MST_PEND;
     int k = sc->kit;
     if (threadIdx.x == 0) {
         mbar_init(&hs.bar, 1);
-        for (int i = 0; i < 12; ++i) mst[i] = sc->mr[k & 1][i];
-        for (int i = 0; i < 5; ++i) pend[i] = sc->pend[i];
-        mst[17] = sc->mr[(k + 1) & 1][MR_BETA_KP1];
+        mr_load(sc, mst, k);
     }
     __syncthreads();
     int phase = 0;
@@ -1037,83 +848,11 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng,
             if (threadIdx.x == 0) part_a[blockIdx.x] = acc;
         }
         if (!grid_sync(gs, limit, flags)) return;
-        // Lanczos step: Q~_{k+1} = W - alpha Q_k - beta_k Q_{k-1},
-        // Z~_{k+1} = Q~_{k+1} / pre (and its FP32 copy); partial Z~_{k+1} . Q~_{k+1}
-        const double alpha = reduce_partials_fused(part_a, gridDim.x);
-        const double beta_k = mst[MR_BETA_KP1], beta_km1 = mst[17];
-        {
-            double* __restrict__ qkp1 = sel3(kb.Q, (k + 1) % 3);
-            const double* __restrict__ qk = sel3(kb.Q, k % 3);
-            const double* __restrict__ qkm1 = sel3(kb.Q, (k + 2) % 3);
-            double* __restrict__ zout = sel2(kb.Z, (k + 1) & 1);
-            float* __restrict__ zfout = sel2(kb.Zf, (k + 1) & 1);
-            double acc = 0;
-            for (int64_t n = t0; n < ng.nn; n += MR_UNROLL * nt) {
-                int64_t nn2[MR_UNROLL];
-                double mm[MR_UNROLL];
-#pragma unroll
-                for (int u = 0; u < MR_UNROLL; ++u) {
-                    const bool in = n + u * nt < ng.nn;
-                    nn2[u] = in ? n + u * nt : n;
-                    mm[u] = in ? gm[nn2[u]] : 0.0;
-                }
-                double pre[MR_UNROLL], qa[MR_UNROLL][3], qb[MR_UNROLL][3], qc[MR_UNROLL][3];
-#pragma unroll
-                for (int u = 0; u < MR_UNROLL; ++u) {
-                    pre[u] = kb.pre[nn2[u]];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const int64_t i = vidx<NPB>(nn2[u], c);
-                        qa[u][c] = qkp1[i];
-                        qb[u][c] = qk[i];
-                        qc[u][c] = qkm1[i];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < MR_UNROLL; ++u) {
-                    if (mm[u] == 0) continue;
-                    float zf[3];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const int64_t i = vidx<NPB>(nn2[u], c);
-                        double q = qa[u][c];
-                        q -= alpha * mr_norm(qb[u][c], beta_k);
-                        q -= beta_k * mr_norm(qc[u][c], beta_km1);
-                        qkp1[i] = q;
-                        const double z = q / pre[u];
-                        zout[i] = z;
-                        zf[c] = (float)z;
-                        acc += z * q;
-                    }
-                    if (zfout) reinterpret_cast<float4*>(zfout)[nn2[u]] = make_float4(zf[0], zf[1], zf[2], 0.f);
-                }
-            }
-            acc = block_sum_fused(acc);
-            if (threadIdx.x == 0) part_b[blockIdx.x] = acc;
-        }
-        if (!grid_sync(gs, limit, flags)) return;
-        const double dz = reduce_partials_fused(part_b, gridDim.x);
-        if (threadIdx.x == 0) {
-            double nx[12] = {};
-            mst[18] = mr_givens(mst, alpha, beta_k, dz, nx, pend);
-            for (int i = 0; i < 12; ++i) mst[i] = nx[i];
-            mst[17] = beta_k;
-        }
-        __syncthreads();
-        const double rnorm = mst[18];
+        double rnorm;
+        if (!mr_lanczos<NPB>(ng, gm, kb, k, mst, part_a, part_b, gs, limit, flags, rnorm)) return;
         ++k;
         const bool go = !(rnorm < local_tol || k >= kmax);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            for (int i = 0; i < 12; ++i) sc->mr[k & 1][i] = mst[i];
-            for (int i = 0; i < 5; ++i) sc->pend[i] = pend[i];
-            sc->rnorm = rnorm;
-            sc->krylov_iters += 1;
-            sc->hvp_count += 1;
-            sc->krylov_bodies += 1;
-            if (nit < 64) sc->kcount[nit] += 1;
-            sc->kit = k;
-            if (!go) sc->kactive = 0;
-        }
+        mr_store(sc, mst, k, nit, rnorm, go);
         if (!go) return;
     }
 }
@@ -1511,38 +1250,6 @@ int launch_newton_tail(const NewtonLaunch& L, cudaStream_t st, cudaGraphConditio
     return ZMPM_OK;
 }
 
-// A persistent Krylov kernel as one cooperative launch of as many CTAs as fit
-// on the device at once (all co-resident, which the grid barrier needs; the
-// launch fails rather than oversubscribes), the grid size found once per
-// kernel.  GridSync must be zero.
-template <class... P, class... A>
-int launch_coop(Ctx* ctx, cudaStream_t st, void (*kern)(P...), A&&... args)
-{
-    int& blocks = ctx->coop_blocks[reinterpret_cast<const void*>(kern)];
-    if (blocks <= 0) {
-        int per_sm = 0, sms = 0;
-        ZMPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FUSED_THREADS, 0));
-        ZMPM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-        blocks = std::min(per_sm * sms, RED_MAX_CTAS);
-        if (blocks <= 0) {
-            ctx->err = "the persistent Krylov kernel does not fit on this device";
-            return ZMPM_CUDA_ERROR;
-        }
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(FUSED_THREADS);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    ZMPM_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
-    ++g_kernel_launches;
-    return ZMPM_OK;
-}
-
 static HvpArgs hvp_args(const Ctx* ctx)
 {
     HvpArgs ha;
@@ -1575,10 +1282,10 @@ int launch_cg_persistent(const NewtonLaunch& L, cudaStream_t st)
             ctx->err = "MIXED CG needs the FP32 copy of p";
             return ZMPM_BAD_ARG;
         }
-        return launch_coop(ctx, st, k_cg_persistent<Lay, float, float>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
+        return launch_coop(ctx, st, RED_MAX_CTAS, k_cg_persistent<Lay, float, float>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
             ctx->spin_limit, flags);
     }
-    return launch_coop(ctx, st, k_cg_persistent<Lay, double, double>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
+    return launch_coop(ctx, st, RED_MAX_CTAS, k_cg_persistent<Lay, double, double>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
         ctx->spin_limit, flags);
 }
 
@@ -1599,9 +1306,9 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
     const long long lim = ctx->spin_limit;
     if (admm) {
         if (ctx->mixed)
-            return launch_coop(ctx, st, k_mr_persistent<Lay, float, double, AdmmOpModel<float>>, L.ng, ha,
+            return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, float, double, AdmmOpModel<float>>, L.ng, ha,
                 AdmmOpModel<float>{ ctx->adm_B.as<float>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
-        return launch_coop(ctx, st, k_mr_persistent<Lay, double, double, AdmmOpModel<double>>, L.ng, ha,
+        return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, double, double, AdmmOpModel<double>>, L.ng, ha,
             AdmmOpModel<double>{ ctx->adm_B.as<double>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
     }
     if (ctx->mixed) {
@@ -1609,11 +1316,11 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
             ctx->err = "MIXED MINRES needs the FP32 copies of Z";
             return ZMPM_BAD_ARG;
         }
-        return launch_coop(ctx, st, k_mr_persistent<Lay, float, float, HvpModel<float>>, L.ng, ha,
+        return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, float, float, HvpModel<float>>, L.ng, ha,
             HvpModel<float>{ ha.pi, ctx->scratch.as<float>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim,
             flags);
     }
-    return launch_coop(ctx, st, k_mr_persistent<Lay, double, double, HvpModel<double>>, L.ng, ha,
+    return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, double, double, HvpModel<double>>, L.ng, ha,
         HvpModel<double>{ ha.pi, ctx->scratch.as<double>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
 }
 
@@ -1856,8 +1563,16 @@ static int admm_impl(Ctx* ctx, const zmpm_solver& s)
     collide(st, ctx->adm_w.as<double>());
     rc = launch_admm_init(ctx, rho);
     if (rc) return rc;
-    ZMPM_CUDA(cudaMemcpyAsync(ctx->adm_pre.p, ctx->gm.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    rc = launch_admm_pre(ctx);
+    // the global operator: the assembled stencil, or matrix-free where the
+    // particles are too sparse for it
+    const bool stencil = stencil_pays(ctx) && stencil_reserve(ctx);
+    ctx->admm_stencil = stencil;
+    if (stencil)
+        rc = launch_stencil_build(ctx);
+    else {
+        ZMPM_CUDA(cudaMemcpyAsync(ctx->adm_pre.p, ctx->gm.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        rc = launch_admm_pre(ctx);
+    }
     if (rc) return rc;
 
     // one ADMM iteration: collision update, local step and the right-hand
@@ -1869,13 +1584,20 @@ static int admm_impl(Ctx* ctx, const zmpm_solver& s)
         if (r) return r;
         r = launch_force_scatter(ctx, ctx->adm_rhs.as<double>());
         if (r) return r;
-        r = launch_admm_op(ctx, ctx->dv.as<double>(), kb.hacc);
+        NodeGeom ns = Lc.ng;
+        if (stencil)
+            r = launch_stencil_start(ctx, kb, Lc.pB, Lc.sc, &ns.parts);
+        else {
+            r = launch_admm_op(ctx, ctx->dv.as<double>(), kb.hacc);
+            if (r) return r;
+            k_admm_start<NPB><<<Lc.nb, ND_THREADS, 0, sm>>>(Lc.ng, ctx->gm.as<double>(), ctx->collided.as<int8_t>(), ctx->proj.as<double>(),
+                ctx->adm_rhs.as<double>(), ctx->dv.as<double>(), kb, Lc.pB, Lc.sc);
+            ++g_kernel_launches;
+        }
         if (r) return r;
-        k_admm_start<NPB><<<Lc.nb, ND_THREADS, 0, sm>>>(Lc.ng, ctx->gm.as<double>(), ctx->collided.as<int8_t>(), ctx->proj.as<double>(),
-            ctx->adm_rhs.as<double>(), ctx->dv.as<double>(), kb, Lc.pB, Lc.sc);
-        k_krylov_start<NPB><<<1, ND_THREADS, 0, sm>>>(Lc.ng, kb, Lc.np, Lc.pB, Lc.sc);
-        g_kernel_launches += 2;
-        r = launch_mr_persistent<NPB>(Lc, sm, true);
+        k_krylov_start<NPB><<<1, ND_THREADS, 0, sm>>>(ns, kb, Lc.np, Lc.pB, Lc.sc);
+        ++g_kernel_launches;
+        r = stencil ? launch_stencil_minres(ctx, Lc.ng, kb, Lc.pA, Lc.pC, Lc.sc, Lc.np.kmax) : launch_mr_persistent<NPB>(Lc, sm, true);
         if (r) return r;
         k_admm_dv_update<NPB><<<Lc.nb, ND_THREADS, 0, sm>>>(Lc.ng, ctx->gm.as<double>(), kb, ctx->vn.as<double>(), ctx->dv.as<double>(),
             ctx->vstar.as<double>(), Lc.sc);
