@@ -54,7 +54,7 @@ struct DBuf {
 struct DevCounters {
     int64_t G, B, N;           // groups, pages, active nodes
     int32_t flags;             // FLAG_*
-    int32_t pad;
+    int32_t max_group;         // particles of the largest group (binning)
     int64_t first_not_max;     // Rankine (reference order): particles whose first eigenvalue is not the largest
     int64_t svd_fp64;          // MIXED: FP32 constitutive updates redone in FP64 (near-degenerate singular values)
 };
@@ -174,7 +174,7 @@ struct Ctx {
     int64_t Pcap = 0;
     DBuf pd, pd_alt, pi, pi_alt;
     DBuf slot_of_id;   // particle index -> slot
-    DBuf base_by_id;   // short4 base node per particle index (binning)
+    DBuf base_by_id;   // short4 base node per particle index, or per old slot (binning)
     DBuf base;         // short4 base node per slot
     DBuf Fn;           // [9][Pcap] F at the start of the Newton solve
     DBuf scratch;      // Hessian scratch [NS][Pcap] in the HVP precision
@@ -188,7 +188,8 @@ struct Ctx {
     // binning
     DBuf keys, keys_alt, flags_i32, scan_i32, scan_scr, radix_scr;
     DBuf group_start, group_page, group_nbr, emit_flag, emit_scan;
-    DBuf page_first, page_block;          // dense page tables
+    DBuf page_first, page_block, page_count; // dense page tables
+    DBuf page_list;                       // occupied pages in any order, then their particle counts (binning)
     DBuf block_page, block_index;         // per page: packed coords, page index
     int64_t G = 0, B = 0, N = 0;
     bool binned = false;
