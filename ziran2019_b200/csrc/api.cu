@@ -474,7 +474,8 @@ int zmpm_destroy(zmpm_ctx* ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DBuf* bufs[] = { &ctx->pd, &ctx->pd_alt, &ctx->pi, &ctx->pi_alt, &ctx->slot_of_id, &ctx->base_by_id, &ctx->base, &ctx->Fn, &ctx->scratch,
         &ctx->frac, &ctx->stress, &ctx->keys, &ctx->keys_alt, &ctx->flags_i32, &ctx->scan_i32, &ctx->scan_scr, &ctx->radix_scr, &ctx->group_start,
-        &ctx->group_page, &ctx->group_nbr, &ctx->emit_flag, &ctx->emit_scan, &ctx->page_first, &ctx->page_block, &ctx->page_count, &ctx->page_list, &ctx->block_page,
+        &ctx->group_page, &ctx->group_nbr, &ctx->emit_flag, &ctx->emit_scan, &ctx->page_first, &ctx->page_block, &ctx->page_count, &ctx->page_list,
+        &ctx->group_cells, &ctx->block_page,
         &ctx->block_index, &ctx->gm, &ctx->gmv, &ctx->vn, &ctx->dv, &ctx->vstar, &ctx->facc, &ctx->res, &ctx->proj, &ctx->collided,
         &ctx->node_idx, &ctx->red, &ctx->scal, &ctx->counters, &ctx->dcolliders, &ctx->adm_F, &ctx->adm_gvn, &ctx->adm_B, &ctx->adm_pre,
         &ctx->adm_rhs, &ctx->adm_w, &ctx->adm_K, &ctx->adm_nbr, &ctx->adj, &ctx->kvf, &ctx->vstarf, &ctx->pfn, &ctx->pfsc, &ctx->gsync };

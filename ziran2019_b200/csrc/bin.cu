@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "xfer.cuh"
 
 namespace zmpm {
 
@@ -300,7 +301,8 @@ __global__ void __launch_bounds__(BIN_THREADS) k_place(const short4* __restrict_
 // element, then by the number of smaller indices in their cell.
 template <class L>
 __global__ void __launch_bounds__(BIN_THREADS) k_order(const int32_t* __restrict__ group_start, const int4* __restrict__ group_page,
-    const uint64_t* __restrict__ pairs, uint64_t* __restrict__ keys, int32_t* __restrict__ old_slot, short4* __restrict__ base)
+    const uint64_t* __restrict__ pairs, uint64_t* __restrict__ keys, int32_t* __restrict__ old_slot, short4* __restrict__ base,
+    int32_t* __restrict__ cells)
 {
     __shared__ uint64_t cell[ORDER_CAP];
     __shared__ int32_t start[L::NPB + 1], fill[L::NPB];
@@ -331,6 +333,8 @@ __global__ void __launch_bounds__(BIN_THREADS) k_order(const int32_t* __restrict
             run += c[k];
         }
         if (threadIdx.x == 31) start[L::NPB] = run;
+        __syncwarp();
+        write_cells<L>(start, g, cells);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -350,6 +354,27 @@ __global__ void __launch_bounds__(BIN_THREADS) k_order(const int32_t* __restrict
         base[at] = make_short4((short)((gp.x << L::XB) | (e >> (L::YB + L::ZB))), (short)((gp.y << L::YB) | ((e >> L::ZB) & (L::BY - 1))),
             (short)((gp.z << L::ZB) | (e & (L::BZ - 1))), 0);
     }
+}
+
+// The cell records of sorted groups (the radix way): one warp per group, cell
+// starts by the heads of equal elements.
+template <class L>
+__global__ void __launch_bounds__(32) k_cells(const int32_t* __restrict__ group_start, const short4* __restrict__ base, int32_t* __restrict__ cells)
+{
+    __shared__ int32_t start[L::NPB + 1];
+    const int g = blockIdx.x, lane = threadIdx.x, s0 = group_start[g], n = group_start[g + 1] - s0;
+    for (int e = lane; e <= L::NPB; e += 32) start[e] = n;
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        const short4 b = base[s0 + i];
+        const int e = (int)L::elem(b.x & (L::BX - 1), b.y & (L::BY - 1), b.z & (L::BZ - 1));
+        atomicMin(&start[e], i);
+    }
+    __syncwarp();
+    if (lane == 0) // an empty cell starts where the next one does
+        for (int e = L::NPB - 1; e >= 0; --e) start[e] = start[e] < start[e + 1] ? start[e] : start[e + 1];
+    __syncwarp();
+    write_cells<L>(start, g, cells);
 }
 
 // New slot i receives the particle of old_slot[i]: every field gathered.
@@ -455,6 +480,9 @@ static int binning_radix(Ctx* ctx)
     ctx->G = G;
 
     ZMPM_CUDA(ctx->group_nbr.ensure(8 * G * sizeof(int32_t)));
+    ZMPM_CUDA(ctx->group_cells.ensure(G * GroupCells<L>::WORDS * sizeof(int32_t)));
+    k_cells<L><<<(unsigned)G, 32, 0, st>>>(ctx->group_start.as<int32_t>(), ctx->base.as<short4>(), ctx->group_cells.as<int32_t>());
+    ++g_kernel_launches;
     ZMPM_CUDA(ctx->emit_flag.ensure(8 * G * sizeof(int32_t)));
     ZMPM_CUDA(ctx->emit_scan.ensure(8 * G * sizeof(int32_t)));
     const int4* gpage = ctx->group_page.as<int4>();
@@ -528,6 +556,7 @@ static int binning_impl(Ctx* ctx)
     ctx->G = G;
     ctx->B = B;
     ZMPM_CUDA(ctx->group_nbr.ensure(8 * G * sizeof(int32_t)));
+    ZMPM_CUDA(ctx->group_cells.ensure(G * GroupCells<L>::WORDS * sizeof(int32_t)));
     ZMPM_CUDA(ctx->block_page.ensure(B * sizeof(int4)));
     ZMPM_CUDA(ctx->block_index.ensure(B * sizeof(uint64_t)));
     int32_t* gstart = ctx->group_start.as<int32_t>();
@@ -536,7 +565,7 @@ static int binning_impl(Ctx* ctx)
     k_rank<<<nblk(32 * G), BIN_THREADS, 0, st>>>(list, list_cnt, (int)G, P, pdims, gstart, gpage, cnt);
     k_place<L><<<nblk(P), BIN_THREADS, 0, st>>>(base_old, P, ctx->pif(PI_ID), pdims, cnt, ctx->keys_alt.as<uint64_t>());
     k_order<L><<<(unsigned)G, BIN_THREADS, 0, st>>>(gstart, gpage, ctx->keys_alt.as<uint64_t>(), ctx->keys.as<uint64_t>(), old_slot,
-        ctx->base.as<short4>());
+        ctx->base.as<short4>(), ctx->group_cells.as<int32_t>());
     k_move<L><<<nblk(P), BIN_THREADS, 0, st>>>(ctx->keys.as<uint64_t>(), old_slot, P, cap, ctx->pd_active, ctx->pd.as<double>(),
         ctx->pd_alt.as<double>(), ctx->pi.as<int32_t>(), ctx->pi_alt.as<int32_t>(), ctx->slot_of_id.as<int32_t>());
     std::swap(ctx->pd, ctx->pd_alt);

@@ -1,6 +1,7 @@
-// Machinery of the fused per-page transfer kernels (Hessian-vector product and
-// the Newton update): one CTA per particle group (the particles whose base node
-// lies in one SPGrid page), in two phases per chunk of the group's particles.
+// Machinery of the fused per-page transfer kernels (Hessian-vector product,
+// Newton update, P2G): a CTA works through pieces of particle groups (the
+// particles whose base node lies in one SPGrid page), each of its warps in two
+// phases per chunk of its own cells' particles.
 //
 //  phase 1 (thread per particle): the particle's B-spline weights, a gradient
 //          gathered from a staged 2x2x2-page window of a grid vector, the
@@ -18,6 +19,8 @@
 // (node (i,j,k) of a particle with base cell (lx,ly,lz) sits at window offset
 // X_i + Y_j + Z_k), so the index arithmetic is one add per node.
 #pragma once
+#include <type_traits>
+
 #include "xfer.cuh"
 
 namespace zmpm {
@@ -232,74 +235,176 @@ __device__ __forceinline__ void gather_gradient_f32(const float* win, const Sten
     }
 }
 
-// Shared state of a fused kernel: the accumulation window, the particle
-// records of the current chunk as 12 arrays of CH values (fractions 0-2, then
-// row r of the scattered matrix at 3 + 3 r .. 5 + 3 r; particle-minor, so a
-// warp's threads of phase 1 write consecutive words), the cell layout of the
-// group and its occupied cells.
-constexpr int REC_FIELDS = 12;
-// stride of one record field: odd, so the rows r of one particle (fields
-// 3 + 3 r + c) fall in different shared-memory banks
-template <int CH>
-constexpr int rec_stride() { return CH + 1; }
-// NF record fields per particle, NC scattered components per node
-template <class L, class T, int CH, int NF = REC_FIELDS, int NC = 3>
-struct ScatterSmem {
-    static constexpr int FS = rec_stride<CH>();
-    __align__(16) T acc[8 * NC * L::NPB];
-    __align__(16) T rec[NF * FS];
-    CellLayout<L> cl;
-    int32_t occ[L::NPB];
-    int32_t nocc;
-    int32_t nbr[8];
+// ------------------------------------------------------ work by particle --
+// The kernels of this family walk the groups as `pieces`: a CTA's share of the
+// particles, cut at group boundaries.  A group costs about K particles' worth
+// of fixed work (window, flush) plus its particles, so group g spans the
+// weights [W(g), W(g + 1)), W(g) = group_start[g] + K g, the total weight is
+// split evenly over the grid and a group that a share boundary cuts becomes two
+// pieces (pieces of one group add to the same nodes).
+struct Piece {
+    int g, g0, s0, s1; // group, its first slot, the piece's slots [s0, s1)
+};
+struct GroupArgs {
+    const int32_t *group_start, *group_nbr, *cells; // cells: GroupCells records, built with the groups
+    int G, K;
+};
+struct Share {
+    const int32_t* gs;
+    int64_t w0, w1;
+    int G, K, first, g;
+
+    __device__ __forceinline__ Share(const GroupArgs& a) : gs(a.group_start), w0(0), w1(0), G(a.G), K(a.K), first(0), g(0)
+    {
+        if (G <= 0) return;
+        const int P = gs[G], n = (int)gridDim.x;
+        // with clearly more CTAs than groups: K at least the share, so that no
+        // share reaches particles of two groups (a second piece would double
+        // the latency of the whole pass)
+        if (2ll * n >= 3ll * G) K = max(K, P / (n - G) + 1);
+        const int64_t total = (int64_t)P + (int64_t)K * G;
+        w0 = total * blockIdx.x / n;
+        w1 = total * (blockIdx.x + 1) / n;
+        int lo = 0, hi = G - 1; // the last group whose weight range starts at or before w0
+        while (lo < hi) {
+            const int m = (lo + hi + 1) >> 1;
+            if ((int64_t)gs[m] + (int64_t)K * m <= w0)
+                lo = m;
+            else
+                hi = m - 1;
+        }
+        first = lo;
+    }
+    __device__ __forceinline__ void rewind() { g = first; }
+    __device__ __forceinline__ bool next(Piece& p)
+    {
+        while (g < G) {
+            const int c = g, g0 = gs[c], n = gs[c + 1] - g0;
+            const int64_t wp = (int64_t)g0 + (int64_t)K * c + K; // weight of the group's first particle
+            if (wp - K >= w1) return false;
+            ++g;
+            const int64_t lo = w0 - wp, hi = w1 - wp;
+            p.g = c;
+            p.g0 = g0;
+            p.s0 = g0 + (int)(lo < 0 ? 0 : (lo > n ? n : lo));
+            p.s1 = g0 + (int)(hi < 0 ? 0 : (hi > n ? n : hi));
+            if (p.s0 < p.s1) return true;
+        }
+        return false;
+    }
 };
 
-// The group's occupied cells, in cell order (after build_cell_layout).
-template <class SM>
-__device__ __forceinline__ void list_occupied(SM& sm)
+// Shared state of a CTA: input windows and accumulation windows in two buffers
+// each (a piece's window arrives during the piece before; its sums are flushed
+// while the next piece accumulates), three buffers of group records (the one
+// being flushed, the running one, the arriving one), and per warp the records
+// of its current chunk of particles, NF arrays of CH values (particle-minor:
+// phase 1's threads write consecutive words).  TX: the input window's type, or
+// void for kernels without one.  CH: what is left of the shared memory that lets
+// CTAS of these run on an SM (227 KB, 1 KB of it reserved per CTA).
+template <class L, class TX>
+struct InputWindow {
+    static constexpr int ELEMS = VecWindow<L::NPB, TX>::ELEMS;
+    using Elem = TX;
+};
+template <class L>
+struct InputWindow<L, void> {
+    static constexpr int ELEMS = 0;
+    using Elem = int32_t;
+};
+template <class L>
+struct MetaBuf {
+    int32_t cells[GroupCells<L>::WORDS];
+    int32_t nbr[8];
+};
+constexpr int FUSED_WARPS = FUSED_THREADS / 32;
+template <class L, class T, class TX, int NF, int NC>
+struct GroupSmem {
+    using W = InputWindow<L, TX>;
+    static constexpr size_t FIXED = 2 * (W::ELEMS * sizeof(typename W::Elem) + 8 * NC * L::NPB * sizeof(T)) + 3 * sizeof(MetaBuf<L>) + 512;
+    static constexpr size_t PER4 = 232448 / 4 - 1024, PER3 = 232448 / 3 - 1024;
+    // four CTAs per SM where the windows leave room for records of a warp's usual share of a page, else three
+    static constexpr int CTAS = FIXED + FUSED_WARPS * NF * 49 * sizeof(T) <= PER4 ? 4 : 3;
+    static constexpr int ROOM = (int)(((CTAS == 4 ? PER4 : PER3) - FIXED) / (FUSED_WARPS * NF * sizeof(T))) - 1;
+    static constexpr int CH = ROOM > 160 ? 160 : ROOM & ~1;
+    static constexpr int FS = CH + 1; // odd: the fields of one particle fall in different banks
+    static_assert(CH >= 32, "a chunk holds at least one particle per lane");
+    alignas(128) typename W::Elem win[2][W::ELEMS ? W::ELEMS : 4];
+    alignas(16) T acc[2][8 * NC * L::NPB];
+    alignas(16) MetaBuf<L> meta[3];
+    alignas(8) uint64_t bar[2];
+    alignas(16) T rec[FUSED_WARPS][NF * FS];
+};
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src)
 {
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int base = 0;
-#pragma unroll
-        for (int c = 0; c < (int)(sizeof(sm.occ) / sizeof(sm.occ[0])); c += 32) {
-            const bool on = sm.cl.cnt[c + lane] > 0;
-            const unsigned m = __ballot_sync(0xffffffffu, on);
-            if (on) sm.occ[base + __popc(m & ((1u << lane) - 1u))] = c + lane;
-            base += __popc(m);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Once per kernel, all threads: the barriers and the accumulation windows.
+template <class SM>
+__device__ __forceinline__ void group_smem_init(SM& sm)
+{
+    if (threadIdx.x == 0) {
+        mbar_init(&sm.bar[0], 1);
+        mbar_init(&sm.bar[1], 1);
+    }
+    constexpr int N = sizeof(sm.acc) / sizeof(sm.acc[0][0]);
+    for (int i = threadIdx.x; i < N; i += FUSED_THREADS) (&sm.acc[0][0])[i] = 0;
+    __syncthreads();
+}
+
+// Starts the transfers of a piece's group record (all threads) and input window
+// (the last warp) into the buffers of piece number ph.
+template <class L, class T, class TX, int NF, int NC>
+__device__ __forceinline__ void group_fetch(GroupSmem<L, T, TX, NF, NC>& sm, const GroupArgs& a, int g, int ph, const TX* x)
+{
+    constexpr int Q = GroupCells<L>::WORDS / 4;
+    static_assert(Q + 2 <= FUSED_THREADS, "one 16-byte copy per thread");
+    MetaBuf<L>& m = sm.meta[ph % 3];
+    const int t = threadIdx.x;
+    if (t < Q)
+        cp_async16(m.cells + 4 * t, a.cells + (int64_t)g * GroupCells<L>::WORDS + 4 * t);
+    else if (t < Q + 2)
+        cp_async16(m.nbr + 4 * (t - Q), a.group_nbr + 8ll * g + 4 * (t - Q));
+    if constexpr (!std::is_void<TX>::value) {
+        using W = VecWindow<L::NPB, TX>;
+        static_assert(W::SLAB % 16 == 0, "bulk copies move multiples of 16 bytes");
+        const int lane = t & 31;
+        if (t >= FUSED_THREADS - 32) {
+            const int32_t nb = lane < 8 ? a.group_nbr[8ll * g + lane] : 0;
+            uint64_t* bar = &sm.bar[ph & 1];
+            if (lane == 0) mbar_expect_tx(bar, 8 * W::SLAB);
+            __syncwarp();
+            if (lane < 8) {
+                // the vector's generic-proxy writes (other CTAs, before a grid barrier) come before the bulk reads
+                asm volatile("fence.proxy.async.global;" ::: "memory");
+                bulk_g2s(&sm.win[ph & 1][lane * W::PAGE], x + (int64_t)nb * W::PAGE, W::SLAB, bar);
+            }
         }
-        if (lane == 0) sm.nocc = base;
     }
 }
 
-// Phase 2 for the chunk of group particles [c0, c1) (group-relative): thread
-// item (row r, occupied cell) adds sum_p row_r(M_p) . grad w_ip * dx to the
-// window for the cell's particles in the chunk (the rows already carry 1/dx).
-// FP32 takes the cell's particles two at a time as packed pairs.
-template <class L, class T, int CH>
-__device__ __forceinline__ void scatter_rows(ScatterSmem<L, T, CH>& sm, int c0, int c1)
-{
-    constexpr int NPB = L::NPB;
-    // items row-major: the threads of a warp hold consecutive cells of one row,
-    // so their window atomics fall in distinct banks
-    const int nocc = sm.nocc, items = 3 * nocc;
-    for (int q = threadIdx.x; q < items; q += blockDim.x) {
-        const int r = q >= nocc ? (q >= 2 * nocc ? 2 : 1) : 0, cidx = q - r * nocc;
-        const int ce = sm.occ[cidx];
-        const int st = sm.cl.start[ce];
-        const int p0 = (st > c0 ? st : c0) - c0;
-        const int e1 = st + sm.cl.cnt[ce];
-        const int p1 = (e1 < c1 ? e1 : c1) - c0;
-        if (p0 >= p1) continue;
-        constexpr int FS = ScatterSmem<L, T, CH>::FS;
-        const T* fr = sm.rec;
-        const T* rrow = sm.rec + (3 + 3 * r) * FS;
-        T a[27];
+// Phase 2 forms.  sum(): a[n] over the particles p0, p0 + 1 (then every `step`
+// pairs) .. of one cell for item row r, from the chunk's records.
+//
+// Rows: sum_p row_r(M_p) . grad w_ip * dx (the rows already carry 1/dx).
+// Records: fractions at 0-2, row r of the scattered matrix at 3 + 3 r ..
+// 5 + 3 r.  FP32 takes particles two at a time as packed pairs.
+template <class T>
+struct RowsScatter {
+    static constexpr int NF = 12, NC = 3;
+    template <int FS>
+    __device__ __forceinline__ static void sum(const T* rec, int r, int p0, int p1, int part, int parts, T a[27])
+    {
+        const T* fr = rec;
+        const T* rrow = rec + (3 + 3 * r) * FS;
         if constexpr (sizeof(T) == 4) {
             float2 a2[27];
 #pragma unroll
             for (int n = 0; n < 27; ++n) a2[n] = f2(0.f);
-            for (int p = p0; p < p1; p += 2) {
+            for (int p = p0 + 2 * part; p < p1; p += 2 * parts) {
                 // an odd last particle pairs with itself at zero weight
                 const int pq = p + 1 < p1 ? p + 1 : p;
                 const float sq = p + 1 < p1 ? 1.f : 0.f;
@@ -325,7 +430,7 @@ __device__ __forceinline__ void scatter_rows(ScatterSmem<L, T, CH>& sm, int c0, 
         else {
 #pragma unroll
             for (int n = 0; n < 27; ++n) a[n] = T(0);
-            for (int p = p0; p < p1; ++p) {
+            for (int p = p0 + part; p < p1; p += parts) {
                 T w[3][3], dw[3][3];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) bspline_all(fr[d * FS + p], w[d], dw[d]);
@@ -341,46 +446,27 @@ __device__ __forceinline__ void scatter_rows(ScatterSmem<L, T, CH>& sm, int c0, 
                     }
             }
         }
-        const int lx = ce >> (L::YB + L::ZB), ly = (ce >> L::ZB) & (L::BY - 1), lz = ce & (L::BZ - 1);
-        const StencilOffsets<L> so(lx, ly, lz);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) atomicAdd(sm.acc + window_scalar<NPB>(so.X[i] + so.Y[j] + so.Z[k], r, 3), a[9 * i + 3 * j + k]);
     }
-}
+};
 
-// Phase 2 of the APIC P2G (particlesToGridHelper, MpmSimulationBase.cpp:563-
-// 608) for the chunk [c0, c1): item (component c, occupied cell) adds, for the
-// cell's particles, w_ip m_p (c = 0) or w_ip (q_r + a_r i + b_r j + c_r k)
-// (c = r + 1, the momentum m (v + C (x_i - x_p)) written affinely in the node
-// offset (i, j, k)) to the window.  Records: fractions at fields 0-2, the mass
-// at 3, row r's (q, a, b, c) at 4 + 4 r .. 7 + 4 r.  FP32 takes the cell's
-// particles two at a time as packed pairs.
-template <class L, class T, int CH>
-__device__ __forceinline__ void scatter_p2g(ScatterSmem<L, T, CH, 16, 4>& sm, int c0, int c1)
-{
-    constexpr int NPB = L::NPB;
-    constexpr int FS = ScatterSmem<L, T, CH, 16, 4>::FS;
-    const int nocc = sm.nocc, items = 4 * nocc;
-    for (int q = threadIdx.x; q < items; q += blockDim.x) {
-        const int c = q / nocc, cidx = q - c * nocc;
-        const int ce = sm.occ[cidx];
-        const int st = sm.cl.start[ce];
-        const int p0 = (st > c0 ? st : c0) - c0;
-        const int e1 = st + sm.cl.cnt[ce];
-        const int p1 = (e1 < c1 ? e1 : c1) - c0;
-        if (p0 >= p1) continue;
-        const T* fr = sm.rec;
-        const T* row = sm.rec + (c == 0 ? 3 : 4 * c) * FS; // mass, or (q, a, b, c) of row c - 1
-        T a[27];
+// APIC P2G (particlesToGridHelper, MpmSimulationBase.cpp:563-608): item
+// (component r, cell) adds w_ip m_p (r = 0) or w_ip (q + a i + b j + c k)
+// (r >= 1, the momentum m (v + C (x_i - x_p)) written affinely in the node
+// offset (i, j, k)).  Records: fractions at 0-2, the mass at 3, (q, a, b, c) of
+// momentum component r - 1 at 4 r .. 4 r + 3.
+template <class T>
+struct P2gScatter {
+    static constexpr int NF = 16, NC = 4;
+    template <int FS>
+    __device__ __forceinline__ static void sum(const T* rec, int r, int p0, int p1, int part, int parts, T a[27])
+    {
+        const T* fr = rec;
+        const T* row = rec + (r == 0 ? 3 : 4 * r) * FS;
         if constexpr (sizeof(T) == 4) {
             float2 a2[27];
 #pragma unroll
             for (int n = 0; n < 27; ++n) a2[n] = f2(0.f);
-            for (int p = p0; p < p1; p += 2) {
+            for (int p = p0 + 2 * part; p < p1; p += 2 * parts) {
                 const int pq = p + 1 < p1 ? p + 1 : p;
                 const float sq = p + 1 < p1 ? 1.f : 0.f;
                 float2 w[3][3], dw[3][3];
@@ -388,7 +474,7 @@ __device__ __forceinline__ void scatter_p2g(ScatterSmem<L, T, CH, 16, 4>& sm, in
                 for (int d = 0; d < 3; ++d) bspline_all2(f2(fr[d * FS + p], fr[d * FS + pq]), w[d], dw[d]);
                 const float2 q0 = f2(row[p], sq * row[pq]);
                 float2 ax = f2(0.f), by = f2(0.f), cz = f2(0.f);
-                if (c != 0) {
+                if (r != 0) {
                     ax = f2(row[FS + p], sq * row[FS + pq]);
                     by = f2(row[2 * FS + p], sq * row[2 * FS + pq]);
                     cz = f2(row[3 * FS + p], sq * row[3 * FS + pq]);
@@ -415,12 +501,12 @@ __device__ __forceinline__ void scatter_p2g(ScatterSmem<L, T, CH, 16, 4>& sm, in
         else {
 #pragma unroll
             for (int n = 0; n < 27; ++n) a[n] = T(0);
-            for (int p = p0; p < p1; ++p) {
+            for (int p = p0 + part; p < p1; p += parts) {
                 T w[3][3], dw[3][3];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) bspline_all(fr[d * FS + p], w[d], dw[d]);
                 const T q0 = row[p];
-                const T ax = c ? row[FS + p] : T(0), by = c ? row[2 * FS + p] : T(0), cz = c ? row[3 * FS + p] : T(0);
+                const T ax = r ? row[FS + p] : T(0), by = r ? row[2 * FS + p] : T(0), cz = r ? row[3 * FS + p] : T(0);
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
 #pragma unroll
@@ -432,14 +518,121 @@ __device__ __forceinline__ void scatter_p2g(ScatterSmem<L, T, CH, 16, 4>& sm, in
                     }
             }
         }
-        const int lx = ce >> (L::YB + L::ZB), ly = (ce >> L::ZB) & (L::BY - 1), lz = ce & (L::BZ - 1);
-        const StencilOffsets<L> so(lx, ly, lz);
+    }
+};
+
+// One warp's part of a piece: the occupied cells whose first particle falls in
+// its quarter of the piece's particles.  Warps do not wait for one another
+// inside a piece; each alternates phase 1 (lane per particle, record into the
+// warp's own shared memory) and phase 2 (lane per (row, cell) item, one shared
+// atomic per node) over its own particles, so one warp's loads overlap
+// another's arithmetic.  When the last round of items leaves half the lanes
+// free, two lanes share an item's particles.
+template <class L, class T, class TX, class Scatter, class Phase1>
+__device__ __forceinline__ void group_warp(GroupSmem<L, T, TX, Scatter::NF, Scatter::NC>& sm, const Piece& pc, int ph, const Phase1& phase1)
+{
+    using SM = GroupSmem<L, T, TX, Scatter::NF, Scatter::NC>;
+    constexpr int NPB = L::NPB, NC = Scatter::NC, FS = SM::FS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t* st = sm.meta[ph % 3].cells; // group-relative first particle of each cell, [NPB + 1]
+    const int nocc = st[GroupCells<L>::NOCC];
+    const uint8_t* occ = reinterpret_cast<const uint8_t*>(st + GroupCells<L>::OCC);
+    const int a0 = pc.s0 - pc.g0, a1 = pc.s1 - pc.g0, n = a1 - a0;
+    const int t0 = a0 + n * warp / FUSED_WARPS, t1 = a0 + n * (warp + 1) / FUSED_WARPS;
+    // the warp's run [lo, hi) of the occupied cells, by their first particle in the piece
+    int lo = 0, hi = 0;
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+    for (int k = 0; k < NPB; k += 32) {
+        bool below0 = false, below1 = false;
+        if (k + lane < nocc) {
+            const int c = occ[k + lane], b = st[c], e = st[c + 1], f = b > a0 ? b : a0;
+            below0 = e <= a0 || f < t0;
+            below1 = e <= a0 || f < t1;
+        }
+        lo += __popc(__ballot_sync(0xffffffffu, below0));
+        hi += __popc(__ballot_sync(0xffffffffu, below1));
+    }
+    if (lo >= hi) return;
+    const int b0 = st[occ[lo]], e1 = st[occ[hi - 1] + 1];
+    const int p_lo = b0 > a0 ? b0 : a0, p_hi = e1 < a1 ? e1 : a1;
+    T* rec = sm.rec[warp];
+    T* acc = sm.acc[ph & 1];
+    const int ncell = hi - lo, items = NC * ncell;
+    for (int c0 = p_lo; c0 < p_hi; c0 += SM::CH) {
+        const int c1 = c0 + SM::CH < p_hi ? c0 + SM::CH : p_hi;
+        __syncwarp();
+        for (int p = c0 + lane; p < c1; p += 32) phase1.template run<FS>(sm.win[ph & 1], (int64_t)(pc.g0 + p), rec + (p - c0));
+        __syncwarp();
+        for (int q0 = 0; q0 < items; q0 += 32) {
+            const int left = items - q0;
+            const int parts = left <= 16 ? 2 : 1, width = parts == 2 ? left : 32; // items of this round
+            const int part = parts == 2 && lane >= width ? 1 : 0;
+            const int q = q0 + lane - part * width;
+            const bool on = q < items && (parts == 1 || lane < 2 * width);
+            // items row-major: the lanes hold consecutive cells of one row, so
+            // their window atomics fall in distinct banks
+            const int r = on ? q / ncell : 0, ce = occ[lo + (on ? q - r * ncell : 0)];
+            const int b = st[ce], e = st[ce + 1];
+            const int p0 = (b > c0 ? b : c0) - c0, p1 = on ? (e < c1 ? e : c1) - c0 : p0;
+            T a[27];
+            Scatter::template sum<FS>(rec, r, p0, p1, part, parts, a);
+            if (parts == 2) {
 #pragma unroll
-            for (int j = 0; j < 3; ++j)
+                for (int m = 0; m < 27; ++m) a[m] += __shfl_down_sync(0xffffffffu, a[m], width);
+            }
+            if (p0 >= p1 || part) continue;
+            const int lx = ce >> (L::YB + L::ZB), ly = (ce >> L::ZB) & (L::BY - 1), lz = ce & (L::BZ - 1);
+            const StencilOffsets<L> so(lx, ly, lz);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) atomicAdd(sm.acc + window_scalar<NPB>(so.X[i] + so.Y[j] + so.Z[k], c, 4), a[9 * i + 3 * j + k]);
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) atomicAdd(acc + window_scalar<NPB>(so.X[i] + so.Y[j] + so.Z[k], r, NC), a[9 * i + 3 * j + k]);
+        }
+    }
+}
+
+// All pieces of the CTA's share: out += the scattered sums (component c < NC0
+// to outa [B][NC0][NPB], the rest to outb).  All threads call it; ph counts the
+// CTA's pieces over the kernel.  One block barrier per piece: it separates the
+// piece's sums from their flush, and the flush (which leaves its buffer zero)
+// from the buffer's next use two pieces later.
+template <class L, class T, class TX, class Scatter, int NC0, class Phase1>
+__device__ __forceinline__ void group_share(GroupSmem<L, T, TX, Scatter::NF, Scatter::NC>& sm, const GroupArgs& a, Share& share, const TX* x,
+    double* __restrict__ outa, double* __restrict__ outb, int32_t* flags, int& ph, const Phase1& phase1)
+{
+    constexpr int NPB = L::NPB, NC = Scatter::NC;
+    Piece cur, nxt;
+    share.rewind();
+    bool have = share.next(cur);
+    if (!have) return;
+    group_fetch(sm, a, cur.g, ph, x);
+    cp_async_wait_all();
+    __syncthreads();
+    while (have) {
+        const bool more = share.next(nxt);
+        if (more) group_fetch(sm, a, nxt.g, ph + 1, x);
+        if constexpr (!std::is_void<TX>::value) mbar_wait_bounded(&sm.bar[ph & 1], (uint32_t)((ph >> 1) & 1), flags);
+        group_warp<L, T, TX, Scatter>(sm, cur, ph, phase1);
+        cp_async_wait_all();
+        __syncthreads();
+        T* acc = sm.acc[ph & 1];
+        const int32_t* nbr = sm.meta[ph % 3].nbr;
+        for (int i = threadIdx.x; i < 8 * NC * NPB; i += FUSED_THREADS) {
+            const T v = acc[i];
+            if (v == T(0)) continue;
+            acc[i] = T(0);
+            const int t = i / (NC * NPB), r = i - t * NC * NPB, c = r / NPB, e = r - c * NPB;
+            const int64_t blk = nbr[t];
+            if (c < NC0)
+                atomicAdd(&outa[(blk * NC0 + c) * NPB + e], (double)v);
+            else
+                atomicAdd(&outb[(blk * (NC - NC0) + (c - NC0)) * NPB + e], (double)v);
+        }
+        cur = nxt;
+        have = more;
+        ++ph;
     }
 }
 

@@ -93,11 +93,8 @@ enum MinresSlot { MR_GC0, MR_GS0, MR_GC1, MR_GS1, MR_GC2, MR_GS2, MR_RHS0, MR_RH
 // State of the bounded grid-wide barrier of a persistent (cooperative) kernel,
 // zeroed before each launch.
 struct GridSync {
-    unsigned count;  // CTAs arrived at the current barrier
-    unsigned pad0[31];
-    unsigned gen;    // barriers completed (polled by the waiting CTAs, on its own 128-byte line)
-    unsigned abort;  // 1 once a CTA's wait gave up
-    unsigned pad1[30];
+    unsigned long long count; // arrivals at all barriers so far; the top bit: a CTA's wait gave up
+    unsigned long long pad[15];
 };
 
 // Field indices of the particle pools.
@@ -188,6 +185,7 @@ struct Ctx {
     // binning
     DBuf keys, keys_alt, flags_i32, scan_i32, scan_scr, radix_scr;
     DBuf group_start, group_page, group_nbr, emit_flag, emit_scan;
+    DBuf group_cells;                     // GroupCells record per group (xfer.cuh)
     DBuf page_first, page_block, page_count; // dense page tables
     DBuf page_list;                       // occupied pages in any order, then their particle counts (binning)
     DBuf block_page, block_index;         // per page: packed coords, page index

@@ -49,39 +49,47 @@ __device__ __forceinline__ T* sel2(T* const (&a)[2], int i) { return i == 0 ? a[
 
 // MINRES keeps its Lanczos vectors Q_j and preconditioned vectors Z_j
 // unnormalised (Minres.h:170-173 divides them by beta_j at the end of
-// iteration j - 1); every reader divides by beta_j, the same rounding as the
-// stored normalised vector.  beta_j = 0 leaves them as they are, as there.
-__device__ __forceinline__ double mr_norm(double v, double beta) { return beta > 0 ? v / beta : v; }
+// iteration j - 1); every reader scales by 1 / beta_j.  beta_j = 0 leaves them
+// as they are, as there.  The node passes multiply by reciprocals formed once
+// per thread: an FP64 division is a chain of about 300 cycles, and the 24 of a
+// thread's two nodes were most of a small scene's operator pass (7.7 of 39 us
+// per iteration at 33k particles).
+__device__ __forceinline__ double mr_scale(double beta) { return beta > 0 ? 1.0 / beta : 1.0; }
 
 // The search direction of iteration j = k - 1 (Minres.h:167-170):
 // M_j = (Z_j - delta M_{j-1} - epsilon M_{j-2}) / gamma, then x += t M_j.
 // The Lanczos step computes its scalars; the vector update runs in the next
 // iteration's operator pass or, after the last iteration, where the solve's x
-// is used (k_newton_step, k_admm_dv_update).
+// is used (k_newton_step, k_admm_dv_update).  M_{-1}, M_{-2} and the first x are
+// zero and not stored: has1, has2 and hasx say which vectors exist.
 struct MrPending {
     const double *z, *m1, *m2;
     double* out;
-    double delta, eps, gamma, t, beta;
-    bool on;
+    double delta, eps, t, ibeta, igamma;
+    bool on, has1, has2, hasx;
 };
 __device__ __forceinline__ MrPending mr_pending(const KrylovBufs& kb, const double* pend, int k)
 {
     MrPending p;
     p.on = k > 0;
+    p.has1 = k > 1;
+    p.has2 = k > 2;
+    p.hasx = k > 1;
     p.z = sel2(kb.Z, (k + 1) & 1);   // Z_{k-1}, unnormalised
     p.m1 = sel3(kb.M, (k + 1) % 3);  // M_{k-2}
     p.m2 = sel3(kb.M, k % 3);        // M_{k-3}
     p.out = sel3(kb.M, (k + 2) % 3); // M_{k-1}
     p.delta = pend[0];
     p.eps = pend[1];
-    p.gamma = pend[2];
+    p.igamma = p.on ? 1.0 / pend[2] : 0.0;
     p.t = pend[3];
-    p.beta = pend[4];                // beta_{k-1}
+    p.ibeta = p.on ? mr_scale(pend[4]) : 0.0; // beta_{k-1}
     return p;
 }
 __device__ __forceinline__ double mr_direction(const MrPending& p, int64_t i)
 {
-    return (mr_norm(p.z[i], p.beta) - p.delta * p.m1[i] - p.eps * p.m2[i]) / p.gamma;
+    const double m1 = p.has1 ? p.m1[i] : 0.0, m2 = p.has2 ? p.m2[i] : 0.0;
+    return (p.z[i] * p.ibeta - p.delta * m1 - p.eps * m2) * p.igamma;
 }
 
 // The Givens update of MINRES iteration k (Minres.h:151-175): from the state
@@ -153,41 +161,39 @@ __device__ __forceinline__ double reduce_partials_fused(const double* part, int 
     return block_sum_fused(s);
 }
 
-// Bounded grid-wide barrier (sense by generation count).  Returns false in
-// every thread of the CTA when this CTA gave up after `limit` polls or another
-// CTA did; the caller then returns.
-__device__ __forceinline__ bool grid_sync(GridSync* gs, long long limit, int32_t* flags)
+// Bounded grid-wide barrier number `epoch` (counted from 0 by every CTA alike):
+// each CTA adds itself to one running count and waits until the count shows all
+// of them, so a barrier is one release and one acquire apart (a separate
+// generation word, written by the last arrival, cost another trip to L2; with
+// its fences 2.3 us on 592 CTAs).  The count's top bit is the abort flag.  Returns false
+// in every thread of the CTA when this CTA gave up after `limit` polls or
+// another CTA did; the caller then returns.
+__device__ __forceinline__ bool grid_sync(GridSync* gs, unsigned& epoch, long long limit, int32_t* flags)
 {
     __shared__ int ok;
+    ++epoch;
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned* vgen = &gs->gen;
-        volatile unsigned* vabort = &gs->abort;
+        constexpr unsigned long long ABORT = 1ull << 63;
+        const unsigned long long target = (unsigned long long)epoch * gridDim.x;
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&gs->count), "l"(1ull) : "memory");
         int good = 1;
-        const unsigned g = *vgen;
-        __threadfence();
-        if (atomicAdd(&gs->count, 1u) == gridDim.x - 1) {
-            gs->count = 0;
-            __threadfence();
-            atomicAdd(&gs->gen, 1u);
-        }
-        else {
-            long long it = 0;
-            while (*vgen == g) {
-                if (*vabort) {
-                    good = 0;
-                    break;
-                }
-                if (++it > limit) {
-                    atomicOr(flags, (int32_t)FLAG_TIMEOUT);
-                    atomicExch(&gs->abort, 1u);
-                    good = 0;
-                    break;
-                }
+        long long it = 0;
+        for (;;) {
+            unsigned long long v;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&gs->count) : "memory");
+            if (v & ABORT) {
+                good = 0;
+                break;
+            }
+            if (v >= target) break;
+            if (++it > limit) {
+                atomicOr(flags, (int32_t)FLAG_TIMEOUT);
+                atomicOr(&gs->count, ABORT);
+                good = 0;
+                break;
             }
         }
-        __threadfence();
-        if (*vabort) good = 0;
         ok = good;
     }
     __syncthreads();
@@ -231,11 +237,13 @@ __device__ __forceinline__ void mr_store(SolverScalars* sc, const double* mst, i
 // a barrier gave up.
 template <int NPB>
 __device__ __forceinline__ bool mr_lanczos(NodeGeom ng, const double* __restrict__ gm, const KrylovBufs& kb, int k, double* mst,
-    const double* part_a, double* part_b, GridSync* gs, long long limit, int32_t* flags, double& rnorm)
+    const double* part_a, double* part_b, GridSync* gs, unsigned& epoch, long long limit, int32_t* flags, double& rnorm)
 {
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     const double alpha = reduce_partials_fused(part_a, gridDim.x);
-    const double beta_k = mst[MR_BETA_KP1], beta_km1 = mst[MST_BETA_KM1];
+    const double beta_k = mst[MR_BETA_KP1];
+    const double ak = alpha * mr_scale(beta_k), bk = beta_k * mr_scale(mst[MST_BETA_KM1]);
+    const bool first = k == 0; // Q_{-1} = 0 is not stored
     // (W may come from other CTAs: ordinary loads, not the read-only path)
     double* qkp1 = sel3(kb.Q, (k + 1) % 3);
     const double* qk = sel3(kb.Q, k % 3);
@@ -261,21 +269,22 @@ __device__ __forceinline__ bool mr_lanczos(NodeGeom ng, const double* __restrict
                 const int64_t i = vidx<NPB>(nn2[u], c);
                 qa[u][c] = qkp1[i];
                 qb[u][c] = qk[i];
-                qc[u][c] = qkm1[i];
+                qc[u][c] = first ? 0.0 : qkm1[i];
             }
         }
 #pragma unroll
         for (int u = 0; u < MR_UNROLL; ++u) {
             if (mm[u] == 0) continue;
             float zf[3];
+            const double ipre = 1.0 / pre[u];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const int64_t i = vidx<NPB>(nn2[u], c);
                 double q = qa[u][c];
-                q -= alpha * mr_norm(qb[u][c], beta_k);
-                q -= beta_k * mr_norm(qc[u][c], beta_km1);
+                q -= ak * qb[u][c];
+                q -= bk * qc[u][c];
                 qkp1[i] = q;
-                const double z = q / pre[u];
+                const double z = q * ipre;
                 zout[i] = z;
                 zf[c] = (float)z;
                 acc += z * q;
@@ -285,7 +294,7 @@ __device__ __forceinline__ bool mr_lanczos(NodeGeom ng, const double* __restrict
     }
     acc = block_sum_fused(acc);
     if (threadIdx.x == 0) part_b[blockIdx.x] = acc;
-    if (!grid_sync(gs, limit, flags)) return false;
+    if (!grid_sync(gs, epoch, limit, flags)) return false;
     const double dz = reduce_partials_fused(part_b, gridDim.x);
     if (threadIdx.x == 0) {
         double nx[12] = {};
@@ -298,37 +307,45 @@ __device__ __forceinline__ bool mr_lanczos(NodeGeom ng, const double* __restrict
     return true;
 }
 
-// A persistent Krylov kernel as one cooperative launch of as many CTAs as fit
-// on the device at once (all co-resident, which the grid barrier needs; the
-// launch fails rather than oversubscribes), the grid size found once per
-// kernel; `useful`: the CTAs the work can occupy (fewer make the barriers
-// cheaper).  GridSync must be zero.
+// A kernel of as many CTAs of FUSED_THREADS threads as fit on the device at
+// once, or `useful` (the CTAs its work can occupy; fewer make barriers cheaper)
+// if that is less; `smem`: its dynamic shared memory.  coop: cooperative, so
+// that all CTAs are co-resident, which the grid barrier needs (the launch fails
+// rather than oversubscribes; GridSync must be zero).  The CTAs that fit are
+// found once per kernel.
 template <class... P, class... A>
-int launch_coop(Ctx* ctx, cudaStream_t st, int64_t useful, void (*kern)(P...), A&&... args)
+int launch_resident(Ctx* ctx, cudaStream_t st, bool coop, int64_t useful, size_t smem, void (*kern)(P...), A&&... args)
 {
     int& blocks = ctx->coop_blocks[reinterpret_cast<const void*>(kern)];
     if (blocks <= 0) {
         int per_sm = 0, sms = 0;
-        ZMPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FUSED_THREADS, 0));
+        if (smem > 0) ZMPM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ZMPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FUSED_THREADS, smem));
         ZMPM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
         blocks = std::min(per_sm * sms, RED_MAX_CTAS);
         if (blocks <= 0) {
-            ctx->err = "the persistent Krylov kernel does not fit on this device";
+            ctx->err = "a kernel does not fit on this device";
             return ZMPM_CUDA_ERROR;
         }
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks, useful)));
     cfg.blockDim = dim3(FUSED_THREADS);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = coop ? 1 : 0;
     ZMPM_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
     ++g_kernel_launches;
     return ZMPM_OK;
 }
+
+// CTAs that a pass over the particles in pieces can occupy: about PIECE_MIN
+// particles' worth of work each.
+constexpr int PIECE_MIN = 64;
+inline int64_t useful_ctas(const Ctx* ctx, int K) { return (ctx->P + (int64_t)K * ctx->G + PIECE_MIN - 1) / PIECE_MIN; }
 
 } // namespace zmpm

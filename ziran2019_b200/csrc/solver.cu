@@ -358,8 +358,9 @@ __global__ void __launch_bounds__(ND_THREADS) k_residual(NodeGeom ng, const doub
 
 // The Newton residual of k_residual fused with the operands of the linear
 // solve's start, in one node pass: r = project(dt m g + dt f - m dv), facc
-// zeroed, x = 0, and from r the Krylov start vectors (CG: r, q = p = r/pre;
-// MINRES: Q0 = r, Z0 = r/pre and its FP32 copy, Q1 = Q2 = M* = Z1 = 0);
+// zeroed, and from r the Krylov start vectors (CG: x = 0, r, q = p = r/pre;
+// MINRES: Q0 = r, Z0 = r/pre and its FP32 copy, Z1 = 0; the vectors of earlier
+// iterations, zero, are not stored);
 // partials of |r|^2/m (computeNorm, BackwardEuler.h:101-140) and of z.r.
 // When k_newton_start then finds the norm converged these vectors go unused.
 template <int NPB>
@@ -382,26 +383,22 @@ __global__ void __launch_bounds__(ND_THREADS, 4) k_residual_start(NodeGeom ng, c
             project3(col, P6, ng.nn, n, r);
             acc += (r[0] * r[0] + r[1] * r[1] + r[2] * r[2]) / m;
         }
+        const double ipre = 1.0 / kb.pre[n];
         for (int k = 0; k < 3; ++k) {
             const int64_t i = vidx<NPB>(n, k);
             const double rv = r[k];
-            const double z = (m != 0) ? rv / kb.pre[n] : 0.0;
-            kb.x[i] = 0;
+            const double z = (m != 0) ? rv * ipre : 0.0;
             if (minres) {
                 kb.Q[0][i] = rv;
-                kb.Q[1][i] = 0;
-                kb.Q[2][i] = 0;
-                kb.M[0][i] = 0;
-                kb.M[1][i] = 0;
-                kb.M[2][i] = 0;
                 kb.Z[0][i] = z;
-                kb.Z[1][i] = 0;
+                kb.Z[1][i] = 0; // massless nodes keep this zero
                 if (kb.Zf[0]) {
                     kb.Zf[0][4 * n + k] = (float)z;
                     kb.Zf[1][4 * n + k] = 0;
                 }
             }
             else {
+                kb.x[i] = 0;
                 kb.r[i] = rv;
                 kb.q[i] = z;
                 kb.p[i] = z;
@@ -548,65 +545,19 @@ __global__ void __launch_bounds__(ND_THREADS) k_apply_A(NodeGeom ng, const doubl
 // loop decision.  The barrier waits are bounded: a CTA that gives up raises
 // FLAG_TIMEOUT and the abort flag, and every CTA returns at its next barrier.
 
-struct HvpArgs {
-    const int32_t *group_start, *group_nbr, *pi;
-    const short4* base;
-    const void *frac, *scr; // in the product's precision
-    int64_t cap;
-    double dx;
-    int G;
-};
-
-// The product of x into out over this CTA's share of the particle groups.  A
-// group's cost is about K particles' worth of fixed work (staging the window,
-// the cell layout, the flush) plus its particles, so group g spans the
-// weights [W(g), W(g + 1)), W(g) = group_start[g] + K g; the total weight is
-// split evenly over the grid and a group whose weight range a share boundary
-// cuts is split into two pieces at the matching particle (pieces of one group
-// add to the same nodes).  K measured on B200 at 1M particles: about 192
-// FP32 particles, 128 FP64 ones (the per-particle work costs more in FP64).
-template <class L, class T, class TX, int CH, class Model>
-__device__ __forceinline__ void hvp_share(HvpSmem<L, T, TX, CH>& hs, const HvpArgs& ha, const Model& model, const TX* x, double* out,
-    int32_t* flags, int& phase)
-{
-    constexpr int PIECE_COST = sizeof(T) == 4 ? 192 : 128;
-    if (ha.G <= 0) return;
-    const int32_t* __restrict__ gs = ha.group_start;
-    const int64_t total = (int64_t)gs[ha.G] + (int64_t)PIECE_COST * ha.G;
-    const int64_t w0 = total * blockIdx.x / gridDim.x, w1 = total * (blockIdx.x + 1) / gridDim.x;
-    if (w0 >= w1) return;
-    int a = 0, b = ha.G - 1; // the last group whose weight range starts at or before w0
-    while (a < b) {
-        const int m = (a + b + 1) >> 1;
-        if ((int64_t)gs[m] + (int64_t)PIECE_COST * m <= w0)
-            a = m;
-        else
-            b = m - 1;
-    }
-    for (int g = a; g < ha.G; ++g) {
-        const int g0 = gs[g], n = gs[g + 1] - g0;
-        const int64_t wp = (int64_t)g0 + (int64_t)PIECE_COST * g + PIECE_COST; // weight of the group's first particle
-        if (wp - PIECE_COST >= w1) break;
-        const int64_t lo = w0 - wp, hi = w1 - wp;
-        const int s0 = g0 + (int)(lo < 0 ? 0 : (lo > n ? n : lo)), s1 = g0 + (int)(hi < 0 ? 0 : (hi > n ? n : hi));
-        if (s0 < s1)
-            hvp_group<L, T, TX, CH>(hs, g, s0, s1, ha.group_nbr, model, ha.cap, ha.base, ha.dx, static_cast<const T*>(ha.frac), x, out, flags,
-                phase++);
-    }
-}
-
 template <class L, class T, class TX>
-__global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng, HvpArgs ha, const double* __restrict__ gm,
+__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_persistent(NodeGeom ng, HvpArgs ha, const double* __restrict__ gm,
     const int8_t* __restrict__ col, const double* __restrict__ P6, double dt2, KrylovBufs kb, double* __restrict__ part_a,
     double* __restrict__ part_b, SolverScalars* __restrict__ sc, int kmax, GridSync* __restrict__ gs, long long limit, int32_t* __restrict__ flags)
 {
     if (sc->newton_done || !sc->kactive) return;
     constexpr int NPB = L::NPB;
-    constexpr int CH = sizeof(T) == 4 ? 512 : 192;
-    __shared__ HvpSmem<L, T, TX, CH> hs;
-    if (threadIdx.x == 0) mbar_init(&hs.bar, 1);
-    __syncthreads();
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    HvpSmem<L, T, TX>& hs = *reinterpret_cast<HvpSmem<L, T, TX>*>(smem_raw);
+    group_smem_init(hs);
+    Share share(ha.ga);
     int phase = 0;
+    unsigned epoch = 0;
     const int nit = sc->nit;
     int k = sc->kit;
     double zTr = sc->mr[k & 1][0];
@@ -620,8 +571,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     for (;;) {
         // the Hessian-vector product of p into hacc
-        hvp_share<L, T, TX, CH>(hs, ha, HvpModel<T>{ ha.pi, static_cast<const T*>(ha.scr), ha.cap }, pin, kb.hacc, flags, phase);
-        if (!grid_sync(gs, limit, flags)) return;
+        hvp_share<L, T, TX>(hs, ha, share, HvpModel<T>{ ha.pi, static_cast<const T*>(ha.scr), ha.cap }, pin, kb.hacc, flags, phase);
+        if (!grid_sync(gs, epoch, limit, flags)) return;
         // tmp = project(m p + dt^2 hacc), hacc = 0; partial p . tmp (BackwardEuler.h:322-351)
         // (two nodes per step, every load issued before the arithmetic, as in
         // k_mr_persistent; massless nodes hold zeros and are not written)
@@ -659,7 +610,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
         }
         acc = block_sum_fused(acc);
         if (threadIdx.x == 0) part_a[blockIdx.x] = acc;
-        if (!grid_sync(gs, limit, flags)) return;
+        if (!grid_sync(gs, epoch, limit, flags)) return;
         // x += alpha p; r -= alpha tmp; q = r / m; partial q . r
         const double alpha = zTr / reduce_partials_fused(part_a, gridDim.x);
         acc = 0;
@@ -683,13 +634,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 if (mm[u] == 0) continue;
+                const double ipre = 1.0 / pre[u];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const int64_t i = vidx<NPB>(nu[u], c);
                     kb.x[i] = xv[u][c] + pv[u][c] * alpha;
                     const double r = rv[u][c] - tv[u][c] * alpha;
                     kb.r[i] = r;
-                    const double q = r / pre[u];
+                    const double q = r * ipre;
                     kb.q[i] = q;
                     acc += q * r;
                 }
@@ -697,7 +649,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
         }
         acc = block_sum_fused(acc);
         if (threadIdx.x == 0) part_b[blockIdx.x] = acc;
-        if (!grid_sync(gs, limit, flags)) return;
+        if (!grid_sync(gs, epoch, limit, flags)) return;
         // beta, p = q + beta p; the loop test of the next iteration
         const double zTr1 = reduce_partials_fused(part_b, gridDim.x);
         const double beta = zTr1 / zTr, rnorm = sqrt(zTr1);
@@ -740,7 +692,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
             if (!go) sc->kactive = 0;
         }
         if (!go) return;
-        if (!grid_sync(gs, limit, flags)) return; // p complete before the next product
+        if (!grid_sync(gs, epoch, limit, flags)) return; // p complete before the next product
     }
 }
 
@@ -761,23 +713,22 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_cg_persistent(NodeGeom ng,
 // complete before the operator pass reads hacc, W before the Lanczos step, and
 // Z~_{k+1} before the next product and the reduction of its norm.
 template <class L, class T, class TX, class Model>
-__global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng, HvpArgs ha, Model model, const double* __restrict__ gm,
+__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_mr_persistent(NodeGeom ng, HvpArgs ha, Model model, const double* __restrict__ gm,
     const int8_t* __restrict__ col, const double* __restrict__ P6, double dt2, KrylovBufs kb, double* __restrict__ part_a,
     double* __restrict__ part_b, SolverScalars* __restrict__ sc, int kmax, GridSync* __restrict__ gs, long long limit, int32_t* __restrict__ flags)
 {
     if (sc->newton_done || !sc->kactive) return;
     constexpr int NPB = L::NPB;
-    constexpr int CH = sizeof(T) == 4 ? 512 : 192;
-    __shared__ HvpSmem<L, T, TX, CH> hs;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    HvpSmem<L, T, TX>& hs = *reinterpret_cast<HvpSmem<L, T, TX>*>(smem_raw);
     __shared__ double mst[MST_N];
     double* const pend = mst + MST_PEND;
     int k = sc->kit;
-    if (threadIdx.x == 0) {
-        mbar_init(&hs.bar, 1);
-        mr_load(sc, mst, k);
-    }
-    __syncthreads();
+    if (threadIdx.x == 0) mr_load(sc, mst, k);
+    group_smem_init(hs);
+    Share share(ha.ga);
     int phase = 0;
+    unsigned epoch = 0;
     const int nit = sc->nit;
     const double local_tol = sc->local_tol;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
@@ -788,15 +739,15 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng,
             zin = reinterpret_cast<const TX*>(sel2(kb.Zf, k & 1));
         else
             zin = reinterpret_cast<const TX*>(sel2(kb.Z, k & 1));
-        hvp_share<L, T, TX, CH>(hs, ha, model, zin, kb.hacc, flags, phase);
-        if (!grid_sync(gs, limit, flags)) return;
+        hvp_share<L, T, TX>(hs, ha, share, model, zin, kb.hacc, flags, phase);
+        if (!grid_sync(gs, epoch, limit, flags)) return;
         // operator pass: the deferred direction of iteration k - 1;
         // W = project(m Z_k + dt2 H Z_k) into Q's slot k + 1; partial Z_k . W
         {
             const double* __restrict__ zk = sel2(kb.Z, k & 1);
             double* __restrict__ w = sel3(kb.Q, (k + 1) % 3);
             const MrPending pd = mr_pending(kb, pend, k);
-            const double beta = mst[MR_BETA_KP1];
+            const double ibeta = mr_scale(mst[MR_BETA_KP1]);
             double acc = 0;
             // MR_UNROLL nodes per step, every load issued before the arithmetic
             // (massless nodes hold zeros in every vector and are not written)
@@ -818,7 +769,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng,
                         zv[u][c] = zk[i];
                         hv[u][c] = kb.hacc[i];
                         mv[u][c] = pd.on ? mr_direction(pd, i) : 0.0;
-                        xv[u][c] = pd.on ? kb.x[i] : 0.0;
+                        xv[u][c] = pd.hasx ? kb.x[i] : 0.0;
                     }
 #pragma unroll
                 for (int u = 0; u < MR_UNROLL; ++u) {
@@ -832,8 +783,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng,
                             pd.out[i] = mv[u][c];
                             kb.x[i] = xv[u][c] + pd.t * mv[u][c];
                         }
-                        z[c] = mr_norm(zv[u][c], beta);
-                        o[c] = m * z[c] + dt2 * mr_norm(hv[u][c], beta);
+                        z[c] = zv[u][c] * ibeta;
+                        o[c] = m * z[c] + dt2 * (hv[u][c] * ibeta);
                         kb.hacc[i] = 0;
                     }
                     project3(col, P6, ng.nn, nn2[u], o);
@@ -847,9 +798,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_persistent(NodeGeom ng,
             acc = block_sum_fused(acc);
             if (threadIdx.x == 0) part_a[blockIdx.x] = acc;
         }
-        if (!grid_sync(gs, limit, flags)) return;
+        if (!grid_sync(gs, epoch, limit, flags)) return;
         double rnorm;
-        if (!mr_lanczos<NPB>(ng, gm, kb, k, mst, part_a, part_b, gs, limit, flags, rnorm)) return;
+        if (!mr_lanczos<NPB>(ng, gm, kb, k, mst, part_a, part_b, gs, epoch, limit, flags, rnorm)) return;
         ++k;
         const bool go = !(rnorm < local_tol || k >= kmax);
         mr_store(sc, mst, k, nit, rnorm, go);
@@ -865,17 +816,20 @@ __global__ void __launch_bounds__(ND_THREADS) k_newton_step(NodeGeom ng, const d
     float4* __restrict__ vstar_f)
 {
     if (sc->newton_done) return;
-    MrPending pd = mr_pending(kb, sc->pend, sc->kit);
-    pd.on = pd.on && minres;
+    const MrPending pd = mr_pending(kb, sc->pend, minres ? sc->kit : 0);
     for (int64_t n = (int64_t)blockIdx.x * ND_THREADS + threadIdx.x; n < ng.nn; n += (int64_t)gridDim.x * ND_THREADS) {
         const bool act = gm[n] != 0;
         double vs[3];
         for (int k = 0; k < 3; ++k) {
             int64_t i = vidx<NPB>(n, k);
-            double step = kb.x[i];
-            if (pd.on) step += pd.t * mr_direction(pd, i);
-            double d = dv[i] + step;
-            dv[i] = d;
+            double d = dv[i];
+            if (act) {
+                // MINRES: x exists from its second iteration on
+                double step = !minres || pd.hasx ? kb.x[i] : 0.0;
+                if (pd.on) step += pd.t * mr_direction(pd, i);
+                d += step;
+                dv[i] = d;
+            }
             vs[k] = act ? vn[i] + d : 0.0;
             vstar[i] = vs[k];
         }
@@ -953,8 +907,8 @@ __global__ void __launch_bounds__(ND_THREADS) k_admm_collide(NodeGeom ng, const 
 }
 
 // Start of dvStep's MINRES from the current dv (Minres.h:73-98): r =
-// project(rhs - (m dv + hacc)), zeroes hacc; Q0 = r, Z0 = r / pre, the other
-// Lanczos vectors and search directions 0, the correction x = 0; partial z.r.
+// project(rhs - (m dv + hacc)), zeroes hacc; Q0 = r, Z0 = r / pre (the vectors of
+// earlier iterations and the correction x, zero, are not stored); partial z.r.
 // The relative tolerance is min(0.5, sqrt(max(residual, 1e-6))) with the
 // reference's constant residual 1 (AdmmSimulationFoam.h:779-782): 0.5.
 template <int NPB>
@@ -976,15 +930,9 @@ __global__ void __launch_bounds__(ND_THREADS) k_admm_start(NodeGeom ng, const do
         for (int k = 0; k < 3; ++k) {
             const int64_t i = vidx<NPB>(n, k);
             const double z = (m != 0) ? r[k] / kb.pre[n] : 0.0;
-            kb.x[i] = 0;
             kb.Q[0][i] = r[k];
-            kb.Q[1][i] = 0;
-            kb.Q[2][i] = 0;
-            kb.M[0][i] = 0;
-            kb.M[1][i] = 0;
-            kb.M[2][i] = 0;
             kb.Z[0][i] = z;
-            kb.Z[1][i] = 0;
+            kb.Z[1][i] = 0; // massless nodes keep this zero
             acc += z * r[k];
         }
     }
@@ -1003,10 +951,13 @@ __global__ void __launch_bounds__(ND_THREADS) k_admm_dv_update(NodeGeom ng, cons
         const bool act = gm[n] != 0;
         for (int k = 0; k < 3; ++k) {
             const int64_t i = vidx<NPB>(n, k);
-            double x = kb.x[i];
-            if (pd.on) x += pd.t * mr_direction(pd, i);
-            const double d = dv[i] + x;
-            dv[i] = d;
+            double d = dv[i];
+            if (act) {
+                double x = pd.hasx ? kb.x[i] : 0.0;
+                if (pd.on) x += pd.t * mr_direction(pd, i);
+                d += x;
+                dv[i] = d;
+            }
             vstar[i] = act ? vn[i] + d : 0.0;
         }
     }
@@ -1250,19 +1201,12 @@ int launch_newton_tail(const NewtonLaunch& L, cudaStream_t st, cudaGraphConditio
     return ZMPM_OK;
 }
 
-static HvpArgs hvp_args(const Ctx* ctx)
+// CTAs that a persistent solve can occupy: by its products or by two nodes per
+// thread of its node passes.
+template <class T>
+int64_t useful_solve(const Ctx* ctx)
 {
-    HvpArgs ha;
-    ha.group_start = ctx->group_start.as<int32_t>();
-    ha.group_nbr = ctx->group_nbr.as<int32_t>();
-    ha.pi = ctx->pi.as<int32_t>();
-    ha.base = ctx->base.as<short4>();
-    ha.frac = ctx->frac.p;
-    ha.scr = ctx->scratch.p;
-    ha.cap = ctx->Pcap;
-    ha.dx = ctx->cfg.dx;
-    ha.G = (int)ctx->G;
-    return ha;
+    return std::max(useful_ctas(ctx, hvp_piece<T>()), (ctx->B * ctx->npb() + 2 * FUSED_THREADS - 1) / (2 * FUSED_THREADS));
 }
 
 // The persistent CG solve (k_cg_persistent) on the Newton operator.
@@ -1271,7 +1215,7 @@ int launch_cg_persistent(const NewtonLaunch& L, cudaStream_t st)
 {
     Ctx* ctx = L.ctx;
     using Lay = typename std::conditional<NPB == 32, Layout244, Layout444>::type;
-    const HvpArgs ha = hvp_args(ctx);
+    const HvpArgs ha = hvp_args(ctx, ctx->mixed ? hvp_piece<float>() : hvp_piece<double>());
     int32_t* flags = &ctx->counters.as<DevCounters>()->flags;
     const double* gm = ctx->gm.as<double>();
     const int8_t* col = ctx->collided.as<int8_t>();
@@ -1282,10 +1226,10 @@ int launch_cg_persistent(const NewtonLaunch& L, cudaStream_t st)
             ctx->err = "MIXED CG needs the FP32 copy of p";
             return ZMPM_BAD_ARG;
         }
-        return launch_coop(ctx, st, RED_MAX_CTAS, k_cg_persistent<Lay, float, float>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
+        return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, float>), k_cg_persistent<Lay, float, float>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
             ctx->spin_limit, flags);
     }
-    return launch_coop(ctx, st, RED_MAX_CTAS, k_cg_persistent<Lay, double, double>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
+    return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_cg_persistent<Lay, double, double>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
         ctx->spin_limit, flags);
 }
 
@@ -1297,7 +1241,7 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
 {
     Ctx* ctx = L.ctx;
     using Lay = typename std::conditional<NPB == 32, Layout244, Layout444>::type;
-    const HvpArgs ha = hvp_args(ctx);
+    const HvpArgs ha = hvp_args(ctx, ctx->mixed ? hvp_piece<float>() : hvp_piece<double>());
     int32_t* flags = &ctx->counters.as<DevCounters>()->flags;
     const double* gm = ctx->gm.as<double>();
     const int8_t* col = ctx->collided.as<int8_t>();
@@ -1306,9 +1250,9 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
     const long long lim = ctx->spin_limit;
     if (admm) {
         if (ctx->mixed)
-            return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, float, double, AdmmOpModel<float>>, L.ng, ha,
+            return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, double>), k_mr_persistent<Lay, float, double, AdmmOpModel<float>>, L.ng, ha,
                 AdmmOpModel<float>{ ctx->adm_B.as<float>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
-        return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, double, double, AdmmOpModel<double>>, L.ng, ha,
+        return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_mr_persistent<Lay, double, double, AdmmOpModel<double>>, L.ng, ha,
             AdmmOpModel<double>{ ctx->adm_B.as<double>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
     }
     if (ctx->mixed) {
@@ -1316,11 +1260,11 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
             ctx->err = "MIXED MINRES needs the FP32 copies of Z";
             return ZMPM_BAD_ARG;
         }
-        return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, float, float, HvpModel<float>>, L.ng, ha,
+        return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, float>), k_mr_persistent<Lay, float, float, HvpModel<float>>, L.ng, ha,
             HvpModel<float>{ ha.pi, ctx->scratch.as<float>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim,
             flags);
     }
-    return launch_coop(ctx, st, RED_MAX_CTAS, k_mr_persistent<Lay, double, double, HvpModel<double>>, L.ng, ha,
+    return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_mr_persistent<Lay, double, double, HvpModel<double>>, L.ng, ha,
         HvpModel<double>{ ha.pi, ctx->scratch.as<double>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
 }
 

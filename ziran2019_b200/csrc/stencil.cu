@@ -57,15 +57,13 @@ __global__ void k_stencil_nbr(const int4* __restrict__ block_page, int B, int px
 template <class L, class T, int CH>
 struct AssembleSmem {
     T rec[9 * (CH + 1)]; // fractions 0-2, B 3-8
-    CellLayout<L> cl;
-    int32_t occ[L::NPB];
-    int32_t nocc;
+    int32_t cells[GroupCells<L>::WORDS];
     int32_t nbr[8];
 };
 
 template <class L, class T, int CH>
 __global__ void __launch_bounds__(FUSED_THREADS) k_stencil_assemble(const int32_t* __restrict__ group_start,
-    const int32_t* __restrict__ group_nbr, int64_t cap, const short4* __restrict__ base, double dx, const T* __restrict__ frac,
+    const int32_t* __restrict__ group_nbr, const int32_t* __restrict__ cells, int64_t cap, double dx, const T* __restrict__ frac,
     const T* __restrict__ B, T* __restrict__ K)
 {
     constexpr int NPB = L::NPB, FS = CH + 1;
@@ -73,8 +71,8 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_stencil_assemble(const int32_
     const int g = blockIdx.x;
     if (threadIdx.x < 8) sm.nbr[threadIdx.x] = group_nbr[8 * g + threadIdx.x];
     const int s0 = group_start[g], n = group_start[g + 1] - s0;
-    build_cell_layout<L>(sm.cl, base, s0, s0 + n);
-    list_occupied(sm);
+    for (int i = threadIdx.x; i < GroupCells<L>::WORDS; i += FUSED_THREADS) sm.cells[i] = cells[(int64_t)g * GroupCells<L>::WORDS + i];
+    const uint8_t* occ = reinterpret_cast<const uint8_t*>(sm.cells + GroupCells<L>::OCC);
     const T inv_dx2 = T((1.0 / dx) * (1.0 / dx));
     for (int c0 = 0; c0 < n; c0 += CH) {
         const int c1 = c0 + CH < n ? c0 + CH : n;
@@ -88,12 +86,11 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_stencil_assemble(const int32_
             for (int k = 0; k < 6; ++k) rc[(3 + k) * FS] = B[(int64_t)k * cap + s] * inv_dx2;
         }
         __syncthreads();
-        const int nocc = sm.nocc;
+        const int nocc = sm.cells[GroupCells<L>::NOCC];
         for (int q = threadIdx.x; q < 27 * nocc; q += blockDim.x) {
-            const int i = q / nocc, ce = sm.occ[q - i * nocc];
-            const int st = sm.cl.start[ce];
+            const int i = q / nocc, ce = occ[q - i * nocc];
+            const int st = sm.cells[ce], e1 = sm.cells[ce + 1];
             const int p0 = (st > c0 ? st : c0) - c0;
-            const int e1 = st + sm.cl.cnt[ce];
             const int p1 = (e1 < c1 ? e1 : c1) - c0;
             if (p0 >= p1) continue;
             const int ix = i / 9, iy = (i / 3) % 3, iz = i % 3;
@@ -272,7 +269,7 @@ __device__ __forceinline__ double own(const StencilSmem<L>& sm, int e, int c)
 
 // Start of dvStep's MINRES from the current dv (Minres.h:73-98), as
 // k_admm_start with the product of dv in the same pass: r = project(rhs -
-// (m dv + K dv)); Q0 = r, Z0 = r / pre, the other vectors 0; partial z . r.
+// (m dv + K dv)); Q0 = r, Z0 = r / pre; partial z . r.
 template <class L, class TK>
 __global__ void __launch_bounds__(FUSED_THREADS, 4) k_stencil_start(int B, const TK* __restrict__ K, const int32_t* __restrict__ nbr,
     const double* __restrict__ gm, const int8_t* __restrict__ col, const double* __restrict__ P6, const double* __restrict__ rhs,
@@ -295,15 +292,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_stencil_start(int B, const
         for (int k = 0; k < 3; ++k) {
             const int64_t i = vidx<NPB>(n, k);
             const double z = (m != 0) ? r[k] / kb.pre[n] : 0.0;
-            kb.x[i] = 0;
             kb.Q[0][i] = r[k];
-            kb.Q[1][i] = 0;
-            kb.Q[2][i] = 0;
-            kb.M[0][i] = 0;
-            kb.M[1][i] = 0;
-            kb.M[2][i] = 0;
             kb.Z[0][i] = z;
-            kb.Z[1][i] = 0;
+            kb.Z[1][i] = 0; // massless nodes keep this zero
             acc += z * r[k];
         }
     }
@@ -330,11 +321,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_stencil(NodeGeom ng, in
     __syncthreads();
     const int nit = sc->nit;
     const double local_tol = sc->local_tol;
+    unsigned epoch = 0;
     for (;;) {
         double* w = sel3(kb.Q, (k + 1) % 3);
         const double* zk = sel2(kb.Z, k & 1);
         const MrPending pd = mr_pending(kb, mst + MST_PEND, k);
-        const double beta = mst[MR_BETA_KP1];
+        const double ibeta = mr_scale(mst[MR_BETA_KP1]);
         double acc = 0;
         for (int b = blockIdx.x; b < B; b += gridDim.x) {
             // the node pass's operands, loaded before the product
@@ -347,7 +339,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_stencil(NodeGeom ng, in
                 for (int c = 0; c < 3; ++c) {
                     const int64_t i = vidx<NPB>(n, c);
                     mv[c] = mr_direction(pd, i);
-                    xv[c] = kb.x[i];
+                    xv[c] = pd.hasx ? kb.x[i] : 0.0;
                 }
             double y[3];
             stencil_page<L, TK>(sm, K, nbr, b, gm, zk, y);
@@ -360,8 +352,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_stencil(NodeGeom ng, in
                     pd.out[i] = mv[c];
                     kb.x[i] = xv[c] + pd.t * mv[c];
                 }
-                z[c] = mr_norm(own<L>(sm, threadIdx.x, c), beta);
-                o[c] = m * z[c] + mr_norm(y[c], beta);
+                z[c] = own<L>(sm, threadIdx.x, c) * ibeta;
+                o[c] = m * z[c] + y[c] * ibeta;
             }
             project3(col, P6, ng.nn, n, o);
 #pragma unroll
@@ -372,9 +364,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_stencil(NodeGeom ng, in
         }
         acc = block_sum_fused(acc);
         if (threadIdx.x == 0) part_a[blockIdx.x] = acc;
-        if (!grid_sync(gs, limit, flags)) return;
+        if (!grid_sync(gs, epoch, limit, flags)) return;
         double rnorm;
-        if (!mr_lanczos<NPB>(ng, gm, kb, k, mst, part_a, part_b, gs, limit, flags, rnorm)) return;
+        if (!mr_lanczos<NPB>(ng, gm, kb, k, mst, part_a, part_b, gs, epoch, limit, flags, rnorm)) return;
         ++k;
         const bool go = !(rnorm < local_tol || k >= kmax);
         mr_store(sc, mst, k, nit, rnorm, go);
@@ -405,7 +397,7 @@ static int stencil_build_impl(Ctx* ctx)
         ctx->page_block.as<int32_t>(), ctx->adm_nbr.as<int32_t>());
     ZMPM_CUDA(cudaMemsetAsync(K, 0, (size_t)nn * STENCIL * sizeof(T), st));
     k_stencil_assemble<L, T, sizeof(T) == 4 ? 512 : 256><<<(unsigned)ctx->G, FUSED_THREADS, 0, st>>>(ctx->group_start.as<int32_t>(),
-        ctx->group_nbr.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<T>(), ctx->adm_B.as<T>(), K);
+        ctx->group_nbr.as<int32_t>(), ctx->group_cells.as<int32_t>(), ctx->Pcap, ctx->cfg.dx, ctx->frac.as<T>(), ctx->adm_B.as<T>(), K);
     k_stencil_pre<L::NPB, T><<<(unsigned)((nn + ND_THREADS - 1) / ND_THREADS), ND_THREADS, 0, st>>>(nn, ctx->gm.as<double>(), K,
         ctx->adm_pre.as<double>());
     g_kernel_launches += 3;
@@ -448,7 +440,7 @@ int launch_stencil_start(Ctx* ctx, const KrylovBufs& kb, double* part, SolverSca
 template <class L, class T>
 static int stencil_minres_impl(Ctx* ctx, const NodeGeom& ng, const KrylovBufs& kb, double* pA, double* pB, SolverScalars* sc, int kmax)
 {
-    return launch_coop(ctx, ctx->stream, (int)ctx->B, k_mr_stencil<L, T>, ng, (int)ctx->B, ctx->adm_K.as<T>(), ctx->adm_nbr.as<int32_t>(),
+    return launch_resident(ctx, ctx->stream, true, ctx->B, 0, k_mr_stencil<L, T>, ng, (int)ctx->B, ctx->adm_K.as<T>(), ctx->adm_nbr.as<int32_t>(),
         ctx->gm.as<double>(), ctx->collided.as<int8_t>(), ctx->proj.as<double>(), kb, pA, pB, sc, kmax, ctx->gsync.as<GridSync>(),
         ctx->spin_limit, &ctx->counters.as<DevCounters>()->flags);
 }

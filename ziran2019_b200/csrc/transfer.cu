@@ -9,15 +9,16 @@
 //            explicit substep's and ADMM's force scatter
 //  k_update_fused  updatePositionBasedState + rasterizeForceToTVStack in one
 //            pass (gather of grad v, F, stress and Hessian scratch, force scatter)
-//  k_hvp_fused  MpmForceBase::addScaledForceDifferential (MpmForceBase.cpp:259-302):
-//            G2P of grad(dv), dS = V0 dP Fn^T, P2G of dS grad w in one pass
-//  k_op_fused  ADMM's global operator in the same one-pass form
+//  k_product  MpmForceBase::addScaledForceDifferential (MpmForceBase.cpp:259-302):
+//            G2P of grad(dv), dS = V0 dP Fn^T, P2G of dS grad w in one pass;
+//            and ADMM's global operator in the same form
 //  k_g2p     gridToParticlesHelper<APIC> (MpmSimulationBase.cpp:906-1016) +
 //            evolveStrain + applyPlasticity (:1018-1030)
 #include "admm.cuh"
 #include "eig3.cuh"
 #include "fused.cuh"
 #include "hvp.cuh"
+#include "krylov.cuh"
 #include "xfer.cuh"
 
 namespace zmpm {
@@ -125,60 +126,61 @@ __global__ void __launch_bounds__(XF_THREADS, 3) k_p2g_reg(const int32_t* __rest
     flush_window<4, 1, NPB>(acc, nbr, gm, gmv);
 }
 
-// APIC P2G as a fused per-page kernel (fused.cuh): phase 1 writes each
-// particle's cell fractions (also to `frac`, for the Newton kernels), its mass
-// and the affine form of its momentum; phase 2 (scatter_p2g) sums them into the
-// window by (component, occupied cell) items.  T: arithmetic (FP32 in MIXED
-// contexts); the window is flushed into the FP64 grid sums.
-template <class L, class T, int CH>
-__global__ void __launch_bounds__(FUSED_THREADS) k_p2g_fused(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    const double* __restrict__ pd, int64_t cap, const short4* __restrict__ base, double dx, double* __restrict__ gm, double* __restrict__ gmv,
-    T* __restrict__ frac)
-{
-    constexpr int NPB = L::NPB;
-    using SM = ScatterSmem<L, T, CH, 16, 4>;
-    __shared__ SM sm;
-    const int g = blockIdx.x;
-    if (threadIdx.x < 8) sm.nbr[threadIdx.x] = group_nbr[8 * g + threadIdx.x];
-    zero_window<4, NPB>(sm.acc);
-    const int s0 = group_start[g], n = group_start[g + 1] - s0;
-    build_cell_layout<L>(sm.cl, base, s0, s0 + n);
-    list_occupied(sm);
-    const double inv_dx = 1.0 / dx;
-    const T tdx = T(dx);
-    for (int c0 = 0; c0 < n; c0 += CH) {
-        const int c1 = c0 + CH < n ? c0 + CH : n;
-        __syncthreads();
-        for (int p = c0 + threadIdx.x; p < c1; p += blockDim.x) {
-            const int64_t s = s0 + p;
-            T* rc = sm.rec + (p - c0);
-            const short4 b = base[s];
-            T fr[3];
+// APIC P2G as a fused kernel (fused.cuh): phase 1 writes each particle's cell
+// fractions (also to `frac`, for the Newton kernels), its mass and the affine
+// form of its momentum; phase 2 (P2gScatter) sums them into the window by
+// (component, occupied cell) items.  T: arithmetic (FP32 in MIXED contexts);
+// the window is flushed into the FP64 grid sums.
+template <class L, class T>
+struct P2gPhase1 {
+    const double* pd;
+    int64_t cap;
+    const short4* base;
+    double inv_dx;
+    T tdx;
+    T* frac;
+
+    template <int FS>
+    __device__ __forceinline__ void run(const void*, int64_t s, T* rc) const
+    {
+        const short4 b = base[s];
+        T fr[3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const double d0 = inv_dx * pd[(PD_X + d) * cap + s] - (double)((&b.x)[d]);
-                fr[d] = (T)d0;
-                frac[d * cap + s] = fr[d];
-                rc[d * SM::FS] = fr[d];
-            }
-            const double mass = pd[PD_M * cap + s];
-            rc[3 * SM::FS] = (T)mass;
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                T mC[3];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) mC[q] = (T)(mass * pd[(PD_C + 3 * r + q) * cap + s]);
-                const T mv = (T)(mass * pd[(PD_V + r) * cap + s]);
-                rc[(4 + 4 * r) * SM::FS] = mv - tdx * (mC[0] * fr[0] + mC[1] * fr[1] + mC[2] * fr[2]);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) rc[(5 + 4 * r + q) * SM::FS] = tdx * mC[q];
-            }
+        for (int d = 0; d < 3; ++d) {
+            const double d0 = inv_dx * pd[(PD_X + d) * cap + s] - (double)((&b.x)[d]);
+            fr[d] = (T)d0;
+            frac[d * cap + s] = fr[d];
+            rc[d * FS] = fr[d];
         }
-        __syncthreads();
-        scatter_p2g(sm, c0, c1);
+        const double mass = pd[PD_M * cap + s];
+        rc[3 * FS] = (T)mass;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            T mC[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) mC[q] = (T)(mass * pd[(PD_C + 3 * r + q) * cap + s]);
+            const T mv = (T)(mass * pd[(PD_V + r) * cap + s]);
+            rc[(4 + 4 * r) * FS] = mv - tdx * (mC[0] * fr[0] + mC[1] * fr[1] + mC[2] * fr[2]);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) rc[(5 + 4 * r + q) * FS] = tdx * mC[q];
+        }
     }
-    __syncthreads();
-    flush_window<4, 1, NPB>(sm.acc, sm.nbr, gm, gmv);
+};
+template <class L, class T>
+using P2gSmem = GroupSmem<L, T, void, P2gScatter<T>::NF, P2gScatter<T>::NC>;
+constexpr int P2G_PIECE = 96; // fixed cost of a piece in particles
+
+template <class L, class T>
+__global__ void __launch_bounds__(FUSED_THREADS, P2gSmem<L, T>::CTAS) k_p2g_fused(GroupArgs ga, const double* __restrict__ pd, int64_t cap,
+    const short4* __restrict__ base, double dx, double* __restrict__ gm, double* __restrict__ gmv, T* __restrict__ frac, int32_t* __restrict__ flags)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    P2gSmem<L, T>& sm = *reinterpret_cast<P2gSmem<L, T>*>(smem_raw);
+    group_smem_init(sm);
+    Share share(ga);
+    int ph = 0;
+    group_share<L, T, void, P2gScatter<T>, 1>(sm, ga, share, nullptr, gm, gmv, flags, ph,
+        P2gPhase1<L, T>{ pd, cap, base, 1.0 / dx, T(dx), frac });
 }
 
 // -------------------------------------------------------------- damage -----
@@ -491,31 +493,19 @@ __global__ void __launch_bounds__(XF_THREADS) k_force(const int32_t* __restrict_
 }
 
 // ------------------------------------------------------- fused products ----
-// The Hessian-vector product (hvp.cuh) as one CTA per particle group (the
-// zmpm_multiply hook; the solves run it inside their persistent kernels).
-template <class L, class T, class TX, int CH>
-__global__ void __launch_bounds__(FUSED_THREADS) k_hvp_fused(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    const int32_t* __restrict__ pi, int64_t cap, const short4* __restrict__ base, double dx, const T* __restrict__ frac,
-    const T* __restrict__ scr, const TX* __restrict__ x, double* __restrict__ out, int32_t* __restrict__ flags)
-{
-    __shared__ HvpSmem<L, T, TX, CH> hs;
-    const int g = blockIdx.x;
-    hvp_group<L, T, TX, CH>(hs, g, group_start[g], group_start[g + 1], group_nbr, HvpModel<T>{ pi, scr, cap }, cap, base, dx, frac, x, out,
-        flags);
-}
-
-// ADMM's global operator (the matrix-free product of dvStep's MINRES,
-// AdmmSimulationFoam.h:167-170 with the B of initMultiplierAndPreconditioner):
-// out += sum_p (grad(x)_p B_p) grad w_ip, one CTA per particle group.
-template <class L, class T, int CH>
-__global__ void __launch_bounds__(FUSED_THREADS) k_op_fused(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    int64_t cap, const short4* __restrict__ base, double dx, const T* __restrict__ frac, const T* __restrict__ B, const double* __restrict__ x,
+// A product (hvp.cuh) as a kernel of its own: the zmpm_multiply hook's Hessian
+// product, and ADMM's global operator out += sum_p (grad(x)_p B_p) grad w_ip
+// (the matrix-free product of dvStep's MINRES, AdmmSimulationFoam.h:167-170).
+template <class L, class T, class TX, class Model>
+__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_product(HvpArgs ha, Model model, const TX* __restrict__ x,
     double* __restrict__ out, int32_t* __restrict__ flags)
 {
-    __shared__ HvpSmem<L, T, double, CH> hs;
-    const int g = blockIdx.x;
-    hvp_group<L, T, double, CH>(hs, g, group_start[g], group_start[g + 1], group_nbr, AdmmOpModel<T>{ B, cap }, cap, base, dx, frac, x, out,
-        flags);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    HvpSmem<L, T, TX>& sm = *reinterpret_cast<HvpSmem<L, T, TX>*>(smem_raw);
+    group_smem_init(sm);
+    Share share(ha.ga);
+    int ph = 0;
+    hvp_share<L, T, TX>(sm, ha, share, model, x, out, flags, ph);
 }
 
 // MpmForceBase::updatePositionBasedState + rasterizeForceToTVStack
@@ -525,91 +515,85 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_op_fused(const int32_t* __res
 // Hessian scratch (updateImplicitState, :68-92); FP32 evaluations of
 // near-degenerate SVDs are redone in FP64.  Phase 2 adds -S_p grad w_ip to
 // facc.  gate as k_stress / k_force.
-template <class L, class T, class TX, int CH>
-__global__ void __launch_bounds__(FUSED_THREADS, 4) k_update_fused(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    const double* __restrict__ pd, const int32_t* __restrict__ pi, int64_t cap, const short4* __restrict__ base, double dx, double dt,
-    const T* __restrict__ frac, const TX* __restrict__ vstar, T* __restrict__ scr, double* __restrict__ facc,
-    const SolverScalars* __restrict__ sc, int32_t* __restrict__ flags, int gate, unsigned long long* __restrict__ svd64)
+template <class L, class T, class TX>
+struct UpdatePhase1 {
+    const double* pd;
+    const int32_t* pi;
+    int64_t cap;
+    const short4* base;
+    const T* frac;
+    T* scr;
+    unsigned long long* svd64;
+    double inv_dx, dt;
+
+    template <int FS>
+    __device__ __forceinline__ void run(const TX* win, int64_t s, T* rc) const
+    {
+        T fr[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) fr[d] = frac[d * cap + s];
+        const short4 b = base[s];
+        const int kind = pi[PI_KIND * cap + s];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) rc[d * FS] = fr[d];
+        const T tinv = T(inv_dx), tdt = T(dt);
+        M3<T> S = m3_zero<T>();
+        if (kind != ZMPM_MODEL_NONE) {
+            T w[3][3], dw[3][3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) bspline_all(fr[d], w[d], dw[d]);
+            const StencilOffsets<L> so(b.x & (L::BX - 1), b.y & (L::BY - 1), b.z & (L::BZ - 1));
+            M3<T> gv;
+            if constexpr (sizeof(T) == 4 && sizeof(TX) == 4)
+                gather_gradient_f32<L>(win, so, w, dw, gv.a);
+            else
+                gather_gradient<L, T, TX>(win, so, w, dw, gv.a);
+            M3<T> Fn, A = m3_identity<T>();
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                Fn.a[q] = (T)pd[(PD_F + q) * cap + s];
+                A.a[q] += tdt * (gv.a[q] * tinv);
+            }
+            const ModelParams mp{ pd[PD_MU * cap + s], pd[PD_LAM * cap + s], pd[PD_KAPPA * cap + s], pd[PD_G * cap + s] };
+            const double V0 = pd[PD_VOL * cap + s];
+            bool degenerate = false;
+            S = model_update<T, T>(kind, mp, (T)V0, m3_mul(A, Fn), Fn, scr, cap, s, sizeof(T) == 4 ? &degenerate : nullptr);
+            if constexpr (sizeof(T) == 4) {
+                if (degenerate) { // FP64 re-evaluation of near-degenerate particles
+                    atomicAdd(svd64, 1ull);
+                    M3<double> Fnd, Ad = m3_identity<double>();
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) {
+                        Fnd.a[q] = pd[(PD_F + q) * cap + s];
+                        Ad.a[q] += dt * ((double)gv.a[q] * inv_dx);
+                    }
+                    S = m3_cast<T>(model_update<double, T>(kind, mp, V0, m3_mul(Ad, Fnd), Fnd, scr, cap, s, nullptr));
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) rc[(3 + 3 * r + c) * FS] = -S(r, c) * tinv;
+    }
+};
+constexpr int UPDATE_PIECE = 64; // fixed cost of a piece in particles
+
+template <class L, class T, class TX>
+__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_update_fused(GroupArgs ga, const double* __restrict__ pd,
+    const int32_t* __restrict__ pi, int64_t cap, const short4* __restrict__ base, double dx, double dt, const T* __restrict__ frac,
+    const TX* __restrict__ vstar, T* __restrict__ scr, double* __restrict__ facc, const SolverScalars* __restrict__ sc,
+    int32_t* __restrict__ flags, int gate, unsigned long long* __restrict__ svd64)
 {
     if (gated_off(sc, gate)) return;
-    constexpr int NPB = L::NPB;
-    __shared__ __align__(128) TX win[VecWindow<NPB, TX>::ELEMS];
-    __shared__ ScatterSmem<L, T, CH> sm;
-    __shared__ __align__(8) uint64_t bar;
-    const int g = blockIdx.x;
-    if (threadIdx.x < 8) sm.nbr[threadIdx.x] = group_nbr[8 * g + threadIdx.x];
-    zero_window<3, NPB>(sm.acc);
-    __syncthreads();
-    stage_vec_window<NPB, TX>(win, vstar, sm.nbr, &bar, flags);
-    const int s0 = group_start[g], n = group_start[g + 1] - s0;
-    build_cell_layout<L>(sm.cl, base, s0, s0 + n);
-    list_occupied(sm);
-    const T inv_dx = T(1.0 / dx);
-    const T tdt = T(dt);
-    for (int c0 = 0; c0 < n; c0 += CH) {
-        const int c1 = c0 + CH < n ? c0 + CH : n;
-        __syncthreads();
-        for (int p = c0 + threadIdx.x; p < c1; p += blockDim.x) {
-            const int64_t s = s0 + p;
-            T* rc = sm.rec + (p - c0);
-            T fr[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                fr[d] = frac[d * cap + s];
-                rc[d * sm.FS] = fr[d];
-            }
-            const int kind = pi[PI_KIND * cap + s];
-            M3<T> S = m3_zero<T>();
-            if (kind != ZMPM_MODEL_NONE) {
-                const short4 b = base[s];
-                T w[3][3], dw[3][3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) bspline_all(fr[d], w[d], dw[d]);
-                const StencilOffsets<L> so(b.x & (L::BX - 1), b.y & (L::BY - 1), b.z & (L::BZ - 1));
-                M3<T> gv;
-                if constexpr (sizeof(T) == 4 && sizeof(TX) == 4)
-                    gather_gradient_f32<L>(win, so, w, dw, gv.a);
-                else
-                    gather_gradient<L, T, TX>(win, so, w, dw, gv.a);
-                M3<T> Fn, A = m3_identity<T>();
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    Fn.a[q] = (T)pd[(PD_F + q) * cap + s];
-                    A.a[q] += tdt * (gv.a[q] * inv_dx);
-                }
-                const ModelParams mp{ pd[PD_MU * cap + s], pd[PD_LAM * cap + s], pd[PD_KAPPA * cap + s], pd[PD_G * cap + s] };
-                const double V0 = pd[PD_VOL * cap + s];
-                bool degenerate = false;
-                S = model_update<T, T>(kind, mp, (T)V0, m3_mul(A, Fn), Fn, scr, cap, s, sizeof(T) == 4 ? &degenerate : nullptr);
-                if constexpr (sizeof(T) == 4) {
-                    if (degenerate) { // FP64 re-evaluation of near-degenerate particles
-                        atomicAdd(svd64, 1ull);
-                        M3<double> Fnd, Ad = m3_identity<double>();
-#pragma unroll
-                        for (int q = 0; q < 9; ++q) {
-                            Fnd.a[q] = pd[(PD_F + q) * cap + s];
-                            Ad.a[q] += dt * ((double)gv.a[q] * (1.0 / dx));
-                        }
-                        S = m3_cast<T>(model_update<double, T>(kind, mp, V0, m3_mul(Ad, Fnd), Fnd, scr, cap, s, nullptr));
-                    }
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) rc[(3 + 3 * r + c) * sm.FS] = -S(r, c) * inv_dx;
-        }
-        __syncthreads();
-        scatter_rows(sm, c0, c1);
-    }
-    __syncthreads();
-    flush_window<3, 3, NPB>(sm.acc, sm.nbr, facc, nullptr);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    HvpSmem<L, T, TX>& sm = *reinterpret_cast<HvpSmem<L, T, TX>*>(smem_raw);
+    group_smem_init(sm);
+    Share share(ga);
+    int ph = 0;
+    group_share<L, T, TX, RowsScatter<T>, 3>(sm, ga, share, vstar, facc, nullptr, flags, ph,
+        UpdatePhase1<L, T, TX>{ pd, pi, cap, base, frac, scr, svd64, 1.0 / dx, dt });
 }
-
-// chunk sizes: the particle records of a chunk fill 24 KB (FP32) / 18 KB (FP64), which keeps
-// the static shared memory of a CTA below 48 KB
-template <class T>
-constexpr int fused_chunk() { return sizeof(T) == 4 ? 512 : 192; }
 
 // ------------------------------------------------------------------ G2P ----
 // MpmSimulationBase::applyPlasticity (MpmSimulationBase.cpp:1018-1030) on one
@@ -822,8 +806,9 @@ static int p2g_impl(Ctx* ctx)
     const int64_t G = ctx->G;
     if (G == 0) return ZMPM_OK;
     if (ctx->mixed)
-        k_p2g_fused<L, float, 384><<<(unsigned)G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(),
-            ctx->pd.as<double>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->gm.as<double>(), ctx->gmv.as<double>(), ctx->frac.as<float>());
+        return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, P2G_PIECE), sizeof(P2gSmem<L, float>), k_p2g_fused<L, float>, group_args(ctx, P2G_PIECE),
+            ctx->pd.as<double>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->gm.as<double>(), ctx->gmv.as<double>(),
+            ctx->frac.as<float>(), &ctx->counters.as<DevCounters>()->flags);
     else
         k_p2g_reg<L, double, 2><<<(unsigned)G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(),
             ctx->pd.as<double>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->gm.as<double>(), ctx->gmv.as<double>(), ctx->frac.as<double>());
@@ -850,11 +835,11 @@ static int update_impl(Ctx* ctx, bool gated)
             if (rc) return rc;
             ctx->vstarf_valid = true;
         }
-        k_update_fused<L, float, float, fused_chunk<float>()><<<(unsigned)G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-            ctx->group_nbr.as<int32_t>(), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->dt,
-            ctx->frac.as<float>(), ctx->vstarf.as<float>(), ctx->scratch.as<float>(), ctx->facc.as<double>(), sc, &dc->flags, gate,
-            reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
-        ++g_kernel_launches;
+        int rc = launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, UPDATE_PIECE), sizeof(HvpSmem<L, float, float>),
+            k_update_fused<L, float, float>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(),
+            ctx->cfg.dx, ctx->dt, ctx->frac.as<float>(), ctx->vstarf.as<float>(), ctx->scratch.as<float>(), ctx->facc.as<double>(), sc, &dc->flags,
+            gate, reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
+        if (rc) return rc;
         if (sc) {
             k_stress<L, double, float><<<(unsigned)G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
                 ctx->group_nbr.as<int32_t>(), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx,
@@ -868,11 +853,10 @@ static int update_impl(Ctx* ctx, bool gated)
         }
     }
     else {
-        k_update_fused<L, double, double, fused_chunk<double>()><<<(unsigned)G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-            ctx->group_nbr.as<int32_t>(), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->dt,
-            ctx->frac.as<double>(), ctx->vstar.as<double>(), ctx->scratch.as<double>(), ctx->facc.as<double>(), sc, &dc->flags, 0,
-            reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
-        ++g_kernel_launches;
+        return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, UPDATE_PIECE), sizeof(HvpSmem<L, double, double>),
+            k_update_fused<L, double, double>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(),
+            ctx->cfg.dx, ctx->dt, ctx->frac.as<double>(), ctx->vstar.as<double>(), ctx->scratch.as<double>(), ctx->facc.as<double>(), sc,
+            &dc->flags, 0, reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
     }
     return ZMPM_OK;
 }
@@ -880,22 +864,19 @@ int launch_update(Ctx* ctx, bool gated) { return ctx->layout == 1 ? update_impl<
 
 // out += dt^-2 (Hessian part of A) x: the fused product, T the context's HVP
 // precision, on an FP64 input vector
+template <class L, class T, class Model>
+static int product_impl(Ctx* ctx, const Model& model, const double* x, double* out)
+{
+    return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, hvp_piece<T>()), sizeof(HvpSmem<L, T, double>), k_product<L, T, double, Model>,
+        hvp_args(ctx, hvp_piece<T>()), model, x, out, &ctx->counters.as<DevCounters>()->flags);
+}
 template <class L>
 static int hvp_impl(Ctx* ctx, const double* x, double* out)
 {
-    const int64_t G = ctx->G;
-    if (G == 0) return ZMPM_OK;
-    DevCounters* dc = ctx->counters.as<DevCounters>();
-    if (ctx->mixed)
-        k_hvp_fused<L, float, double, fused_chunk<float>()><<<(unsigned)G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-            ctx->group_nbr.as<int32_t>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<float>(),
-            ctx->scratch.as<float>(), x, out, &dc->flags);
-    else
-        k_hvp_fused<L, double, double, fused_chunk<double>()><<<(unsigned)G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-            ctx->group_nbr.as<int32_t>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<double>(),
-            ctx->scratch.as<double>(), x, out, &dc->flags);
-    ++g_kernel_launches;
-    return ZMPM_OK;
+    if (ctx->G == 0) return ZMPM_OK;
+    const int32_t* pi = ctx->pi.as<int32_t>();
+    if (ctx->mixed) return product_impl<L, float>(ctx, HvpModel<float>{ pi, ctx->scratch.as<float>(), ctx->Pcap }, x, out);
+    return product_impl<L, double>(ctx, HvpModel<double>{ pi, ctx->scratch.as<double>(), ctx->Pcap }, x, out);
 }
 
 int launch_hvp(Ctx* ctx, const double* x, double* out, bool fp32)
@@ -930,17 +911,8 @@ int launch_force_scatter(Ctx* ctx, double* out, bool mls)
 template <class L>
 static int admm_op_impl(Ctx* ctx, const double* x, double* out)
 {
-    DevCounters* dc = ctx->counters.as<DevCounters>();
-    if (ctx->mixed)
-        k_op_fused<L, float, fused_chunk<float>()><<<(unsigned)ctx->G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-            ctx->group_nbr.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<float>(), ctx->adm_B.as<float>(), x, out,
-            &dc->flags);
-    else
-        k_op_fused<L, double, fused_chunk<double>()><<<(unsigned)ctx->G, FUSED_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-            ctx->group_nbr.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<double>(), ctx->adm_B.as<double>(), x,
-            out, &dc->flags);
-    ++g_kernel_launches;
-    return ZMPM_OK;
+    if (ctx->mixed) return product_impl<L, float>(ctx, AdmmOpModel<float>{ ctx->adm_B.as<float>(), ctx->Pcap }, x, out);
+    return product_impl<L, double>(ctx, AdmmOpModel<double>{ ctx->adm_B.as<double>(), ctx->Pcap }, x, out);
 }
 int launch_admm_op(Ctx* ctx, const double* x, double* out)
 {

@@ -216,4 +216,33 @@ __device__ __forceinline__ void build_cell_layout(CellLayout<L>& cl, const short
     __syncthreads();
 }
 
+// Per group, built with the groups and kept for the substep: the first particle
+// of each of the page's cells (relative to the group's first slot) and the end,
+// the number of occupied cells, and their elements in order (bytes).
+template <class L>
+struct GroupCells {
+    static constexpr int NOCC = L::NPB + 1, OCC = L::NPB + 2, WORDS = (L::NPB + 2 + L::NPB / 4 + 3) & ~3;
+};
+// One warp writes group g's record from its cell starts [NPB + 1].
+template <class L>
+__device__ __forceinline__ void write_cells(const int32_t* start, int g, int32_t* __restrict__ cells)
+{
+    const int lane = threadIdx.x & 31;
+    int32_t* rec = cells + (int64_t)g * GroupCells<L>::WORDS;
+    uint8_t* occ = reinterpret_cast<uint8_t*>(rec + GroupCells<L>::OCC);
+    int n = 0;
+#pragma unroll
+    for (int c = 0; c < L::NPB; c += 32) {
+        const int b = start[c + lane], e = start[c + lane + 1];
+        rec[c + lane] = b;
+        const unsigned m = __ballot_sync(0xffffffffu, e > b);
+        if (e > b) occ[n + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(c + lane);
+        n += __popc(m);
+    }
+    if (lane == 0) {
+        rec[L::NPB] = start[L::NPB];
+        rec[GroupCells<L>::NOCC] = n;
+    }
+}
+
 } // namespace zmpm
