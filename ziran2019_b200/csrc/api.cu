@@ -6,7 +6,10 @@
 #include <cstring>
 #include <cstdlib>
 #include <limits>
+#include <mutex>
 #include <new>
+#include <system_error>
+#include <thread>
 
 #include "internal.cuh"
 #include "models.cuh"
@@ -27,6 +30,71 @@ cudaError_t d2h_sync(Ctx* ctx, void* dst, const void* src, size_t bytes)
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
     if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(ctx->stream);
+}
+
+// Device -> caller's memory of a finished array, complete on return.  A plain
+// copy to pageable memory runs at 6 GB/s here (one thread of the driver copies,
+// and takes the page faults of a fresh destination); arrays of a few MB and
+// more go through two pinned blocks instead, one filling over PCIe while
+// threads empty the other.  192 MB (x, v, C, F of 1M particles) into fresh
+// memory: 13-33 -> 12 ms, by host.  The blocks belong to the process, because
+// pinning 8 MB takes about 10 ms: made for the first transfer that wants them,
+// freed with the last context, used by one thread at a time (another thread's
+// transfer meanwhile takes the plain copy).
+constexpr size_t PIN_BLOCK = 4 << 20, PIN_FROM = 2 << 20;
+constexpr int PIN_THREADS = 8;
+struct PinBlocks {
+    std::mutex m;
+    void* p = nullptr;
+    int contexts = 0;
+};
+PinBlocks g_pin;
+
+void copy_threaded(char* dst, const char* src, size_t bytes)
+{
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int n = (int)std::min<size_t>(std::min<size_t>(PIN_THREADS, hw ? hw : 1), bytes / (256 << 10) + 1);
+    std::thread t[PIN_THREADS];
+    const size_t per = ((bytes / n) + 4095) & ~(size_t)4095;
+    int started = 0;
+    for (int i = 1; i < n; ++i) {
+        const size_t a = std::min(bytes, per * i), b = i + 1 == n ? bytes : std::min(bytes, per * (i + 1));
+        if (a >= b) continue;
+        try {
+            t[started] = std::thread([=] { std::memcpy(dst + a, src + a, b - a); });
+            ++started;
+        }
+        catch (const std::system_error&) { // no thread to be had: this one copies
+            std::memcpy(dst + a, src + a, b - a);
+        }
+    }
+    std::memcpy(dst, src, n == 1 ? bytes : std::min(bytes, per));
+    for (int i = 0; i < started; ++i) t[i].join();
+}
+
+cudaError_t copy_out(Ctx* ctx, void* dst, const void* src, size_t bytes)
+{
+    std::unique_lock<std::mutex> lock(g_pin.m, std::defer_lock);
+    if (bytes < PIN_FROM || !lock.try_lock()) return d2h_sync(ctx, dst, src, bytes);
+    if (!g_pin.p && cudaHostAlloc(&g_pin.p, 2 * PIN_BLOCK, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError(); // no pinned memory: the plain copy
+        g_pin.p = nullptr;
+        return d2h_sync(ctx, dst, src, bytes);
+    }
+    char* block[2] = { static_cast<char*>(g_pin.p), static_cast<char*>(g_pin.p) + PIN_BLOCK };
+    const size_t n = (bytes + PIN_BLOCK - 1) / PIN_BLOCK;
+    auto size = [&](size_t k) { return std::min(PIN_BLOCK, bytes - k * PIN_BLOCK); };
+    cudaError_t e = cudaMemcpyAsync(block[0], src, size(0), cudaMemcpyDeviceToHost, ctx->stream);
+    for (size_t k = 0; k < n && e == cudaSuccess; ++k) {
+        e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) break;
+        if (k + 1 < n)
+            e = cudaMemcpyAsync(block[(k + 1) & 1], static_cast<const char*>(src) + (k + 1) * PIN_BLOCK, size(k + 1), cudaMemcpyDeviceToHost,
+                ctx->stream);
+        copy_threaded(static_cast<char*>(dst) + k * PIN_BLOCK, block[k & 1], size(k));
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(ctx->stream); // nothing may still write the blocks
+    return e;
 }
 
 int64_t bitlen(uint64_t v)
@@ -266,13 +334,26 @@ __global__ void k_fields_from_host(const double* __restrict__ in, int ncomp, int
     const int64_t s = slot_of_id[i];
     for (int c = 0; c < ncomp; ++c) field[c * cap + s] = in[i * ncomp + c];
 }
-__global__ void k_fields_to_host(double* __restrict__ out, int ncomp, int64_t P, int64_t cap, const int32_t* __restrict__ slot_of_id,
-    const double* __restrict__ field)
+template <class T>
+__global__ void k_fields_to_host(T* __restrict__ out, int ncomp, int64_t P, int64_t cap, const int32_t* __restrict__ slot_of_id,
+    const T* __restrict__ field)
 {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     const int64_t s = slot_of_id[i];
     for (int c = 0; c < ncomp; ++c) out[i * ncomp + c] = field[c * cap + s];
+}
+
+// mu, lambda and kappa of the particles lo .. lo + n - 1 (st: mu, then lambda).
+__global__ void k_set_lame(const double* __restrict__ st, int64_t n, int64_t lo, int64_t cap, const int32_t* __restrict__ slot_of_id,
+    double* __restrict__ pd)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t s = slot_of_id[lo + i];
+    pd[PD_MU * cap + s] = st[i];
+    pd[PD_LAM * cap + s] = st[n + i];
+    pd[PD_KAPPA * cap + s] = __dadd_rn(__dmul_rn(0.666666, st[i]), st[n + i]); // as the host rounds it
 }
 
 int device_set(Ctx* ctx, const double* x, const double* v, const double* C, const double* F)
@@ -300,27 +381,40 @@ int device_set(Ctx* ctx, const double* x, const double* v, const double* C, cons
     return ZMPM_OK;
 }
 
+// Fields [f, f + ncomp) of the double pool to a host array in particle-index
+// order.  The pool must be on the device and the fields active.
+int get_field(Ctx* ctx, int f, int ncomp, double* dst)
+{
+    const int64_t P = ctx->P;
+    if (P == 0 || !dst) return ZMPM_OK;
+    ZMPM_CUDA(ctx->stage.ensure((size_t)ncomp * P * sizeof(double)));
+    k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, ctx->stream>>>(ctx->stage.as<double>(), ncomp, P, ctx->Pcap,
+        ctx->slot_of_id.as<int32_t>(), ctx->pdf(f));
+    ++g_kernel_launches;
+    ZMPM_CUDA(cudaGetLastError());
+    ZMPM_CUDA(copy_out(ctx, dst, ctx->stage.p, (size_t)ncomp * P * sizeof(double)));
+    return ZMPM_OK;
+}
+int get_field(Ctx* ctx, int f, int32_t* dst)
+{
+    const int64_t P = ctx->P;
+    if (P == 0 || !dst) return ZMPM_OK;
+    ZMPM_CUDA(ctx->stage.ensure(P * sizeof(int32_t)));
+    k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, ctx->stream>>>(ctx->stage.as<int32_t>(), 1, P, ctx->Pcap,
+        ctx->slot_of_id.as<int32_t>(), ctx->pif(f));
+    ++g_kernel_launches;
+    ZMPM_CUDA(cudaGetLastError());
+    ZMPM_CUDA(copy_out(ctx, dst, ctx->stage.p, P * sizeof(int32_t)));
+    return ZMPM_OK;
+}
+
 int device_get(Ctx* ctx, double* x, double* v, double* C, double* F)
 {
-    const int64_t P = ctx->P, cap = ctx->Pcap;
-    if (P == 0) return ZMPM_OK;
-    ZMPM_CUDA(ctx->stage.ensure(24 * P * sizeof(double)));
-    double* st = ctx->stage.as<double>();
-    double* dst[4] = { x, v, C, F };
-    const int nc[4] = { 3, 3, 9, 9 };
-    const int fld[4] = { PD_X, PD_V, PD_C, PD_F };
-    int64_t off = 0;
-    for (int a = 0; a < 4; ++a) {
-        if (!dst[a]) continue;
-        k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, ctx->stream>>>(st + off, nc[a], P, cap, ctx->slot_of_id.as<int32_t>(),
-            ctx->pdf(fld[a]));
-        ++g_kernel_launches;
-        ZMPM_CUDA(cudaMemcpyAsync(dst[a], st + off, nc[a] * P * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        off += nc[a] * P;
-    }
-    ZMPM_CUDA(cudaGetLastError());
-    ZMPM_CUDA(cudaStreamSynchronize(ctx->stream));
-    return ZMPM_OK;
+    int rc = get_field(ctx, PD_X, 3, x);
+    if (!rc) rc = get_field(ctx, PD_V, 3, v);
+    if (!rc) rc = get_field(ctx, PD_C, 9, C);
+    if (!rc) rc = get_field(ctx, PD_F, 9, F);
+    return rc;
 }
 
 int check_ready(Ctx* ctx)
@@ -463,6 +557,10 @@ int zmpm_create(const zmpm_config* cfg, zmpm_ctx** out)
     cudaMemset(ctx->scal.p, 0, sizeof(SolverScalars));
     // the context's stream does not order itself after the legacy stream's memsets
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail(e);
+    {
+        std::lock_guard<std::mutex> lock(g_pin.m);
+        ++g_pin.contexts; // given back in zmpm_destroy
+    }
     *out = ctx;
     return ZMPM_OK;
 }
@@ -484,6 +582,13 @@ int zmpm_destroy(zmpm_ctx* ctx)
     for (auto* v : { &ctx->ckpt_pd, &ctx->ckpt_pi, &ctx->ckpt_sid })
         for (auto& b : *v) b.release();
     ctx->stage.release();
+    {
+        std::lock_guard<std::mutex> lock(g_pin.m);
+        if (--g_pin.contexts == 0 && g_pin.p) {
+            cudaFreeHost(g_pin.p);
+            g_pin.p = nullptr;
+        }
+    }
     for (cudaEvent_t e : ctx->hvp_ev) cudaEventDestroy(e);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -583,8 +688,24 @@ int zmpm_set_lame(zmpm_ctx* ctx, int64_t lo, int64_t hi, const double* mu, const
 {
     if (!ctx || !mu || !lambda || lo < 0 || hi > ctx->P || lo > hi) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    int rc = begin_edit(ctx);
-    if (rc) return rc;
+    if (ctx->uploaded) { // the three parameters alone, on the device
+        const int64_t n = hi - lo;
+        if (n > 0) {
+            ZMPM_CUDA(ctx->stage.ensure(2 * n * sizeof(double)));
+            double* st = ctx->stage.as<double>();
+            ZMPM_CUDA(cudaMemcpyAsync(st, mu, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+            ZMPM_CUDA(cudaMemcpyAsync(st + n, lambda, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+            k_set_lame<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(st, n, lo, ctx->Pcap, ctx->slot_of_id.as<int32_t>(),
+                ctx->pd.as<double>());
+            ++g_kernel_launches;
+            ZMPM_CUDA(cudaGetLastError());
+            ZMPM_CUDA(cudaStreamSynchronize(ctx->stream));
+        }
+        ctx->binned = false;
+        ctx->implicit_ready = false;
+        ctx->phase = 0; // an edit ends a substep split into phases
+        return ZMPM_OK;
+    }
     for (int64_t i = lo; i < hi; ++i) {
         ctx->hmu[i] = mu[i - lo];
         ctx->hlam[i] = lambda[i - lo];
@@ -669,8 +790,7 @@ int zmpm_get_log_jp(zmpm_ctx* ctx, double* log_jp)
 {
     if (!ctx || !log_jp) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    int rc = download(ctx);
-    if (rc) return rc;
+    if (ctx->uploaded) return get_field(ctx, PD_LOGJP, 1, log_jp);
     std::memcpy(log_jp, ctx->hlogjp.data(), ctx->P * sizeof(double));
     return ZMPM_OK;
 }
@@ -695,8 +815,7 @@ int zmpm_get_damage(zmpm_ctx* ctx, double* c)
 {
     if (!ctx || !c) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    int rc = download(ctx);
-    if (rc) return rc;
+    if (ctx->uploaded) return get_field(ctx, PD_PF_C, 1, c);
     for (int64_t i = 0; i < ctx->P; ++i) c[i] = ctx->hpfc[i];
     return ZMPM_OK;
 }
@@ -760,6 +879,14 @@ int zmpm_get_phase_field(zmpm_ctx* ctx, double* c, double* H, double* pf_Fp, dou
 {
     if (!ctx) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
+    if (ctx->uploaded && ctx->pd_active >= PD_PF_END) {
+        int rc = get_field(ctx, PD_PF_C, 1, c);
+        if (!rc) rc = get_field(ctx, PD_PF_H, 1, H);
+        if (!rc) rc = get_field(ctx, PD_PF_FP, 1, pf_Fp);
+        if (!rc) rc = get_field(ctx, PD_PF_VOL, 1, vol);
+        return rc;
+    }
+    // the solve's own fields are not on the device: their host values stand
     int rc = download(ctx);
     if (rc) return rc;
     for (int64_t i = 0; i < ctx->P; ++i) {
@@ -811,8 +938,7 @@ int zmpm_get_viscoelastic_strain(zmpm_ctx* ctx, double* Fe)
 {
     if (!ctx || !Fe) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    int rc = download(ctx);
-    if (rc) return rc;
+    if (ctx->uploaded && ctx->pd_active == PD_FIELDS) return get_field(ctx, PD_FE, 9, Fe);
     std::memcpy(Fe, ctx->hFe.data(), 9 * ctx->P * sizeof(double));
     return ZMPM_OK;
 }
@@ -895,8 +1021,10 @@ int zmpm_get_plastic_state(zmpm_ctx* ctx, double* ys, int32_t* broken)
 {
     if (!ctx) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    int rc = download(ctx);
-    if (rc) return rc;
+    if (ctx->uploaded) {
+        int rc = get_field(ctx, PD_YS, 1, ys);
+        return rc ? rc : get_field(ctx, PI_BROKEN, broken);
+    }
     for (int64_t i = 0; i < ctx->P; ++i) {
         if (ys) ys[i] = ctx->hys[i];
         if (broken) broken[i] = ctx->hbroken[i];
@@ -1270,7 +1398,7 @@ int zmpm_adjoint_substep(zmpm_ctx* ctx, double dt, const zmpm_solver* s, double 
             k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, sm>>>(stg + off, nc[a], P, cap, ctx->slot_of_id.as<int32_t>(),
                 aj + (int64_t)fld[a] * cap);
             ++g_kernel_launches;
-            ZMPM_CUDA(cudaMemcpyAsync(dst[a], stg + off, nc[a] * P * sizeof(double), cudaMemcpyDeviceToHost, sm));
+            ZMPM_CUDA(copy_out(ctx, dst[a], stg + off, nc[a] * P * sizeof(double)));
             off += nc[a] * P;
         }
         if (gE) {
