@@ -54,24 +54,29 @@ ZMPM_HD void hencky_diag(T mu, T lambda, const T s[3], T dE[3], T ddE[3][3])
     for (int d = 0; d < 3; ++d) L[d] = log(fabs(s[d]));
     const T sum_log = L[0] + L[1] + L[2];
     const T g = T(2) * mu + lambda;
+    // one division per singular value (nine quotients otherwise, each a chain of about 300 cycles in FP64)
+    const T r[3] = { T(1) / s[0], T(1) / s[1], T(1) / s[2] };
 #pragma unroll
-    for (int d = 0; d < 3; ++d) dE[d] = (T(2) * mu * L[d] + lambda * sum_log) / s[d];
-    ddE[0][0] = (g * (T(1) - L[0]) - lambda * (L[1] + L[2])) / (s[0] * s[0]);
-    ddE[1][1] = (g * (T(1) - L[1]) - lambda * (L[0] + L[2])) / (s[1] * s[1]);
-    ddE[2][2] = (g * (T(1) - L[2]) - lambda * (L[0] + L[1])) / (s[2] * s[2]);
-    ddE[0][1] = ddE[1][0] = lambda / (s[0] * s[1]);
-    ddE[0][2] = ddE[2][0] = lambda / (s[0] * s[2]);
-    ddE[1][2] = ddE[2][1] = lambda / (s[1] * s[2]);
+    for (int d = 0; d < 3; ++d) dE[d] = (T(2) * mu * L[d] + lambda * sum_log) * r[d];
+    ddE[0][0] = (g * (T(1) - L[0]) - lambda * (L[1] + L[2])) * (r[0] * r[0]);
+    ddE[1][1] = (g * (T(1) - L[1]) - lambda * (L[0] + L[2])) * (r[1] * r[1]);
+    ddE[2][2] = (g * (T(1) - L[2]) - lambda * (L[0] + L[1])) * (r[2] * r[2]);
+    ddE[0][1] = ddE[1][0] = lambda * (r[0] * r[1]);
+    ddE[0][2] = ddE[2][0] = lambda * (r[0] * r[2]);
+    ddE[1][2] = ddE[2][1] = lambda * (r[1] * r[2]);
 }
 
 // Eigenvalues of a symmetric 3x3 matrix by cyclic Jacobi rotations (Golub &
-// Van Loan, Matrix Computations, 8.5.2); at most 50 sweeps.
+// Van Loan, Matrix Computations, 8.5.2); at most 50 sweeps.  The sweeps end
+// once the off-diagonal norm is below 1e-20 of the diagonal's: by Weyl's
+// inequality it moves no eigenvalue by more (running on until it underflows to
+// zero takes about twice the sweeps).
 template <class T>
 ZMPM_HD void sym3_eig(T A[3][3], T ev[3])
 {
     for (int sweep = 0; sweep < 50; ++sweep) {
         const T off = A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2];
-        if (off == T(0)) break;
+        if (off <= T(1e-40) * (A[0][0] * A[0][0] + A[1][1] * A[1][1] + A[2][2] * A[2][2])) break;
 #pragma unroll
         for (int p = 0; p < 2; ++p)
 #pragma unroll
@@ -267,22 +272,22 @@ ZMPM_HD void dp_project_sigma_derivative(T mu, T lambda, T alpha, T cohesion, co
         }
 }
 
-// The viscous map in singular values and its derivative, AdmmSimulationFoam.h:583-595.
+// The viscous map in singular values and its derivative, AdmmSimulationFoam.h:
+// 583-595 (a, b: viscous_coefficients).
 template <class T>
-ZMPM_HD void viscous_sigma(T mu, T lambda, T vd, T vv, T dt, const T zi[3], T zp[3], T D[3][3])
+ZMPM_HD void viscous_sigma(T a, T b, const T zi[3], T zp[3], T D[3][3])
 {
-    T a, b;
-    viscous_coefficients(mu, lambda, vd, vv, dt, a, b);
     T et[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) et[d] = log(fabs(zi[d]));
     const T t = et[0]; // `epsilon_trial.trace()` of a 3-vector, as in viscous_return
 #pragma unroll
     for (int d = 0; d < 3; ++d) zp[d] = exp(a * (et[d] - b * t));
+    const T iz[3] = { T(1) / zi[0], T(1) / zi[1], T(1) / zi[2] };
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) D[r][c] = zp[r] * a * ((r == c ? T(1) / zi[c] : T(0)) - b * (T(1) / zi[c]));
+        for (int c = 0; c < 3; ++c) D[r][c] = zp[r] * a * ((r == c ? iz[c] : T(0)) - b * iz[c]);
 }
 
 enum AdmmLocalMode { ADMM_ELASTIC = 0, ADMM_VON_MISES = 1, ADMM_VISCOUS = 2, ADMM_DRUCKER_PRAGER = 3 };
@@ -305,6 +310,8 @@ ZMPM_D M3<T> admm_local_solve(const M3<T>& FDb, const M3<T>& Fcur, T vol, T coef
     const M3<T> W = m3_Tmul(U, m3_mul(Fcur, V));
     T zi[3] = { W(0, 0), W(1, 1), W(2, 2) };
     const T mu = (T)p.mu, lambda = (T)p.lambda;
+    T va = T(0), vb = T(0);
+    if (mode == ADMM_VISCOUS) viscous_coefficients(mu, lambda, (T)p.vd, (T)p.vv, dt, va, vb);
     for (int j = 0; j < iters; ++j) {
         T zp[3], D[3][3];
         if (mode == ADMM_VON_MISES)
@@ -312,7 +319,7 @@ ZMPM_D M3<T> admm_local_solve(const M3<T>& FDb, const M3<T>& Fcur, T vol, T coef
         else if (mode == ADMM_DRUCKER_PRAGER)
             dp_project_sigma_derivative(mu, lambda, (T)p.alpha, (T)p.cohesion, zi, zp, D);
         else if (mode == ADMM_VISCOUS)
-            viscous_sigma(mu, lambda, (T)p.vd, (T)p.vv, dt, zi, zp, D);
+            viscous_sigma(va, vb, zi, zp, D);
         else {
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
@@ -333,10 +340,10 @@ ZMPM_D M3<T> admm_local_solve(const M3<T>& FDb, const M3<T>& Fcur, T vol, T coef
             for (int c = 0; c < 3; ++c) Pm(r, c) = vol * (ddE[r][0] * D[0][c] + ddE[r][1] * D[1][c] + ddE[r][2] * D[2][c]) + (r == c ? coeff : T(0));
         // step = P^-1 (-g) with P^-1 = adj(P) / det(P)
         const M3<T> C = m3_cofactor(Pm);
-        const T det = Pm(0, 0) * C(0, 0) + Pm(0, 1) * C(0, 1) + Pm(0, 2) * C(0, 2);
+        const T idet = T(-1) / (Pm(0, 0) * C(0, 0) + Pm(0, 1) * C(0, 1) + Pm(0, 2) * C(0, 2));
         T step[3];
 #pragma unroll
-        for (int r = 0; r < 3; ++r) step[r] = (C(0, r) / det) * (-g[0]) + (C(1, r) / det) * (-g[1]) + (C(2, r) / det) * (-g[2]);
+        for (int r = 0; r < 3; ++r) step[r] = (C(0, r) * g[0] + C(1, r) * g[1] + C(2, r) * g[2]) * idet;
 #pragma unroll
         for (int d = 0; d < 3; ++d) zi[d] += step[d];
         if (sqrt(step[0] * step[0] + step[1] * step[1] + step[2] * step[2]) < tol) break;
