@@ -450,7 +450,12 @@ int upload_colliders(Ctx* ctx, double time, int slot)
         }
         d.radius = c.radius;
         quat_to_R(c.rotation, d.R);
+        if (c.shape == ZMPM_HALF_SPACE) {
+            const double nn = std::sqrt(c.b[0] * c.b[0] + c.b[1] * c.b[1] + c.b[2] * c.b[2]);
+            for (int k = 0; k < 3; ++k) d.b[k] = c.b[k] / nn;
+        }
         d.s = c.scale + time * c.scale_velocity;
+        d.ios = 1 / d.s;
         d.dsdt = c.scale_velocity;
     }
     ZMPM_CUDA(cudaMemcpyAsync(ctx->dcolliders.as<DevCollider>() + (size_t)slot * MAX_COLLIDERS, h.data(), n * sizeof(DevCollider),
@@ -1042,10 +1047,9 @@ static int delete_phase_field_particles(zmpm_ctx* ctx)
 }
 
 // Kernels of one Newton loop body when the solve runs as a graph: the update
-// (MIXED: the FP32 pass and the gated FP64 stress / force pair, one of which
-// returns at once), residual with the Krylov start vectors, Newton check with
-// the Krylov start, the persistent linear solve, step, advance.
-static int64_t newton_body_launches(const zmpm_ctx* ctx) { return ctx->mixed ? 8 : 6; }
+// (MIXED: its FP32 and FP64 forms, one of which returns at once), the persistent
+// solve with the iteration's residual, check and step, advance.
+static int64_t newton_body_launches(const zmpm_ctx* ctx) { return ctx->mixed ? 4 : 3; }
 
 static int begin_implicit_impl(zmpm_ctx* ctx, double dt, bool damage = true)
 {

@@ -60,7 +60,7 @@ __device__ __forceinline__ double mr_scale(double beta) { return beta > 0 ? 1.0 
 // M_j = (Z_j - delta M_{j-1} - epsilon M_{j-2}) / gamma, then x += t M_j.
 // The Lanczos step computes its scalars; the vector update runs in the next
 // iteration's operator pass or, after the last iteration, where the solve's x
-// is used (k_newton_step, k_admm_dv_update).  M_{-1}, M_{-2} and the first x are
+// is used (newton_step, k_admm_dv_update).  M_{-1}, M_{-2} and the first x are
 // zero and not stored: has1, has2 and hasx say which vectors exist.
 struct MrPending {
     const double *z, *m1, *m2;
@@ -214,6 +214,12 @@ __device__ __forceinline__ void mr_load(const SolverScalars* sc, double* mst, in
     for (int i = 0; i < 12; ++i) mst[i] = sc->mr[k & 1][i];
     for (int i = 0; i < 5; ++i) mst[MST_PEND + i] = sc->pend[i];
     mst[MST_BETA_KM1] = sc->mr[(k + 1) & 1][MR_BETA_KP1];
+}
+__device__ __forceinline__ void mr_init(double* mst, double rnorm) // one thread: the state before iteration 0
+{
+    for (int i = 0; i < MST_N; ++i) mst[i] = 0;
+    mst[MR_GC0] = mst[MR_GC1] = mst[MR_GC2] = 1;
+    mst[MR_RHS0] = mst[MR_BETA_KP1] = rnorm;
 }
 // CTA 0 stores the state after an iteration (k counts it already).
 __device__ __forceinline__ void mr_store(SolverScalars* sc, const double* mst, int k, int nit, double rnorm, bool go)

@@ -36,8 +36,7 @@ int launch_g2p(Ctx* ctx, bool plastic);
 __device__ bool collider_inside(const DevCollider& c, const double X[3], double N[3], double* phi_out = nullptr)
 {
     if (c.shape == ZMPM_HALF_SPACE) {
-        double nn = sqrt(c.b[0] * c.b[0] + c.b[1] * c.b[1] + c.b[2] * c.b[2]);
-        double n[3] = { c.b[0] / nn, c.b[1] / nn, c.b[2] / nn };
+        const double* n = c.b;
         double phi = n[0] * (X[0] - c.a[0]) + n[1] * (X[1] - c.a[1]) + n[2] * (X[2] - c.a[2]);
         if (phi <= 0) {
             if (phi_out) *phi_out = phi;
@@ -94,7 +93,7 @@ __device__ bool collider_resolve(const DevCollider& c, const double x[3], double
 {
     if (c.type == ZMPM_GHOST) return false;
     double xb[3] = { x[0] - c.t[0], x[1] - c.t[1], x[2] - c.t[2] };
-    double ios = 1 / c.s;
+    const double ios = c.ios;
     double X[3];
     for (int i = 0; i < 3; ++i) X[i] = (c.R[i] * xb[0] + c.R[3 + i] * xb[1] + c.R[6 + i] * xb[2]) * ios;
     double N[3];
@@ -128,7 +127,7 @@ __device__ bool collider_resolve(const DevCollider& c, const double x[3], double
 __device__ bool collider_query_world(const DevCollider& c, const double x[3], double& phi, double n[3])
 {
     double xb[3] = { x[0] - c.t[0], x[1] - c.t[1], x[2] - c.t[2] };
-    double ios = 1 / c.s;
+    const double ios = c.ios;
     double X[3];
     for (int i = 0; i < 3; ++i) X[i] = (c.R[i] * xb[0] + c.R[3 + i] * xb[1] + c.R[6 + i] * xb[2]) * ios;
     double N[3];
@@ -143,7 +142,7 @@ __device__ bool collider_boundary(const DevCollider& c, const double x[3], doubl
 {
     if (c.type == ZMPM_GHOST) return false;
     double xb[3] = { x[0] - c.t[0], x[1] - c.t[1], x[2] - c.t[2] };
-    double ios = 1 / c.s;
+    const double ios = c.ios;
     double X[3];
     for (int i = 0; i < 3; ++i) X[i] = (c.R[i] * xb[0] + c.R[3 + i] * xb[1] + c.R[6 + i] * xb[2]) * ios;
     double N[3];
@@ -232,7 +231,8 @@ __global__ void __launch_bounds__(ND_THREADS) k_grid_init(NodeGeom ng, const dou
         double P[6] = { 1, 0, 0, 1, 0, 1 };
         if (m != 0) {
             ++local;
-            for (int k = 0; k < 3; ++k) v[k] = gmv[vidx<NPB>(n, k)] / m;
+            const double im = 1.0 / m;
+            for (int k = 0; k < 3; ++k) v[k] = gmv[vidx<NPB>(n, k)] * im;
             const int4 bp = block_page[b];
             const int lx = e >> (L::YB + L::ZB), ly = (e >> L::ZB) & (L::BY - 1), lz = e & (L::BZ - 1);
             double xi[3] = { (bp.x * L::BX + lx) * dx, (bp.y * L::BY + ly) * dx, (bp.z * L::BZ + lz) * dx };
@@ -291,9 +291,9 @@ __global__ void __launch_bounds__(ND_THREADS) k_grid_explicit(NodeGeom ng, const
         int8_t c = 0;
         if (m != 0) {
             ++local;
-            const double dt_over_mi = dt / m;
+            const double im = 1.0 / m, dt_over_mi = dt * im;
             for (int k = 0; k < 3; ++k) {
-                v[k] = gmv[vidx<NPB>(n, k)] / m;
+                v[k] = gmv[vidx<NPB>(n, k)] * im;
                 vi[k] = v[k] + g[k] * dt + facc[vidx<NPB>(n, k)] * dt_over_mi;
             }
             const int4 bp = block_page[b];
@@ -354,114 +354,6 @@ __global__ void __launch_bounds__(ND_THREADS) k_residual(NodeGeom ng, const doub
     }
     double s = block_sum(acc);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// The Newton residual of k_residual fused with the operands of the linear
-// solve's start, in one node pass: r = project(dt m g + dt f - m dv), facc
-// zeroed, and from r the Krylov start vectors (CG: x = 0, r, q = p = r/pre;
-// MINRES: Q0 = r, Z0 = r/pre and its FP32 copy, Z1 = 0; the vectors of earlier
-// iterations, zero, are not stored);
-// partials of |r|^2/m (computeNorm, BackwardEuler.h:101-140) and of z.r.
-// When k_newton_start then finds the norm converged these vectors go unused.
-template <int NPB>
-__global__ void __launch_bounds__(ND_THREADS, 4) k_residual_start(NodeGeom ng, const double* __restrict__ gm, double* __restrict__ facc,
-    const double* __restrict__ dv, const int8_t* __restrict__ col, const double* __restrict__ P6, double gx, double gy, double gz, double dt,
-    KrylovBufs kb, int minres, double* __restrict__ part_norm, double* __restrict__ part_zr, const SolverScalars* __restrict__ sc)
-{
-    if (sc->newton_done) return;
-    double acc = 0, zr = 0;
-    const double g[3] = { gx, gy, gz };
-    for (int64_t n = (int64_t)blockIdx.x * ND_THREADS + threadIdx.x; n < ng.nn; n += (int64_t)gridDim.x * ND_THREADS) {
-        const double m = gm[n];
-        double r[3] = { 0, 0, 0 };
-        for (int k = 0; k < 3; ++k) {
-            const int64_t i = vidx<NPB>(n, k);
-            if (m != 0) r[k] = dt * g[k] * m + dt * facc[i] - (dt / dt) * m * dv[i];
-            facc[i] = 0;
-        }
-        if (m != 0) {
-            project3(col, P6, ng.nn, n, r);
-            acc += (r[0] * r[0] + r[1] * r[1] + r[2] * r[2]) / m;
-        }
-        const double ipre = 1.0 / kb.pre[n];
-        for (int k = 0; k < 3; ++k) {
-            const int64_t i = vidx<NPB>(n, k);
-            const double rv = r[k];
-            const double z = (m != 0) ? rv * ipre : 0.0;
-            if (minres) {
-                kb.Q[0][i] = rv;
-                kb.Z[0][i] = z;
-                kb.Z[1][i] = 0; // massless nodes keep this zero
-                if (kb.Zf[0]) {
-                    kb.Zf[0][4 * n + k] = (float)z;
-                    kb.Zf[1][4 * n + k] = 0;
-                }
-            }
-            else {
-                kb.x[i] = 0;
-                kb.r[i] = rv;
-                kb.q[i] = z;
-                kb.p[i] = z;
-                if (kb.pf) kb.pf[4 * n + k] = (float)z;
-            }
-            zr += z * rv;
-        }
-    }
-    const double s0 = block_sum(acc);
-    const double s1 = block_sum(zr);
-    if (threadIdx.x == 0) {
-        part_norm[blockIdx.x] = s0;
-        part_zr[blockIdx.x] = s1;
-    }
-}
-
-// Newton check (NewtonsMethod.h:48-61) and, unless converged, the start of
-// the linear solve (k_krylov_start's scalars).  One CTA.
-template <int NPB>
-__global__ void __launch_bounds__(ND_THREADS) k_newton_start(NodeGeom ng, NewtonParams np, const double* __restrict__ part_norm,
-    const double* __restrict__ part_zr, SolverScalars* __restrict__ sc)
-{
-    if (sc->newton_done) return;
-    const double norm = sqrt(reduce_partials(part_norm, ng.parts));
-    const bool done = (norm < np.tol) || !(norm == norm);
-    const double dotv = reduce_partials(part_zr, ng.parts);
-    if (threadIdx.x != 0) return;
-    if (sc->nit == 0) sc->res_initial = norm;
-    // MIXED: a norm that did not halve means FP32 stress round-off now
-    // dominates the residual; the rest of the solve evaluates it in FP64, and
-    // this iteration takes no step (the residual is re-evaluated first)
-    const bool stall = np.escalate && !done && !sc->fp64_res && sc->nit > 0 && !(norm <= 0.5 * sc->res_final);
-    if (stall) sc->fp64_res = 1;
-    sc->skip_step = stall ? 1 : 0;
-    sc->res_final = norm;
-    if (done) {
-        sc->newton_done = 1;
-        sc->converged = (norm == norm) ? 1 : 0;
-        sc->kactive = 0;
-        return;
-    }
-    const double mx = norm > np.tol ? norm : np.tol;
-    const double rel0 = np.tol_scale * sqrt(mx);
-    const double rel = rel0 < 0.5 ? rel0 : 0.5;
-    sc->rel_tol = rel;
-    // Minres.h:73-98, ConjugateGradient.h:108-117
-    const double rnorm = sqrt(dotv);
-    const double lt = fmin(rel * rnorm, np.abs_tol);
-    const bool active = !(rnorm < lt) && np.kmax > 0 && !stall;
-    sc->rnorm = rnorm;
-    sc->local_tol = lt;
-    sc->kit = 0;
-    sc->kactive = active ? 1 : 0;
-    if (np.minres) {
-        double* mr = sc->mr[0];
-        mr[MR_GC0] = mr[MR_GC1] = mr[MR_GC2] = 1;
-        mr[MR_GS0] = mr[MR_GS1] = mr[MR_GS2] = 0;
-        mr[MR_RHS0] = rnorm;
-        mr[MR_RHS1] = 0;
-        mr[MR_BETA_KP1] = rnorm;
-    }
-    else
-        sc->mr[0][0] = dotv; // CG keeps zTrk double-buffered in mr[parity][0]
 }
 
 // Initial preconditioned norm and local tolerance (Minres.h:73-98,
@@ -545,12 +437,159 @@ __global__ void __launch_bounds__(ND_THREADS) k_apply_A(NodeGeom ng, const doubl
 // loop decision.  The barrier waits are bounded: a CTA that gives up raises
 // FLAG_TIMEOUT and the abort flag, and every CTA returns at its next barrier.
 
-template <class L, class T, class TX>
-__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_persistent(NodeGeom ng, HvpArgs ha, const double* __restrict__ gm,
+// What the persistent solve of a Newton iteration does besides the linear
+// solve: the residual and the Newton check before it, the step after it.
+struct NewtonArgs {
+    NewtonParams np;
+    double* facc;
+    double* dv;
+    const double* vn;
+    double* vstar;
+    float4* vstar_f;      // MIXED: the FP32 copy, else null
+    double* part_norm;
+    double g[3];
+};
+// The linear solve's start, the same in every CTA.
+struct SolveStart {
+    bool active;
+    double rnorm, local_tol, zr;
+};
+
+// Start of a Newton iteration over the grid, ending in a grid barrier: the
+// residual r = project(dt m g + dt f - m dv) with f = facc (BackwardEuler.h:101-
+// 124), facc zeroed, the Krylov start vectors (CG: x = 0, r, q = p = r/m;
+// MINRES: Q0 = r, Z0 = r/m and its FP32 copy, Z1 = 0; the vectors of earlier
+// iterations, zero, are not stored), the norm sqrt(sum |r|^2/m) (computeNorm,
+// :125-140), then the Newton check (NewtonsMethod.h:48-61) and the solve's
+// tolerance (Minres.h:73-98, ConjugateGradient.h:108-117), which every CTA
+// forms alike; CTA 0 stores them.  As separate kernels the pass, the check and
+// the step cost 21 us per iteration at 33k particles (mostly latency).  Returns
+// false when the barrier gave up.
+template <int NPB>
+__device__ __forceinline__ bool newton_begin(NodeGeom ng, const NewtonArgs& na, const double* __restrict__ gm, const int8_t* __restrict__ col,
+    const double* __restrict__ P6, const KrylovBufs& kb, SolverScalars* sc, GridSync* gs, unsigned& epoch, long long limit, int32_t* flags,
+    SolveStart& out)
+{
+    const NewtonParams& np = na.np;
+    // read before the barrier, after which CTA 0 writes them (volatile: the
+    // compiler may not move the reads to their use)
+    const volatile SolverScalars* vsc = sc;
+    const int nit = vsc->nit, was_fp64 = vsc->fp64_res;
+    const double last = vsc->res_final, dt = np.dt;
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    double acc = 0;
+    for (int64_t n = t0; n < ng.nn; n += nt) {
+        const double m = gm[n];
+        double f[3], d[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int64_t i = vidx<NPB>(n, c);
+            f[c] = na.facc[i];
+            d[c] = na.dv[i];
+        }
+        double r[3] = { 0, 0, 0 }, z[3] = { 0, 0, 0 };
+        if (m != 0) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) r[c] = dt * na.g[c] * m + dt * f[c] - m * d[c];
+            project3(col, P6, ng.nn, n, r);
+            const double im = 1.0 / m;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) z[c] = r[c] * im;
+            acc += r[0] * z[0] + r[1] * z[1] + r[2] * z[2];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int64_t i = vidx<NPB>(n, c);
+            na.facc[i] = 0;
+            if (np.minres) {
+                kb.Q[0][i] = r[c];
+                kb.Z[0][i] = z[c];
+                kb.Z[1][i] = 0; // massless nodes keep this zero
+            }
+            else {
+                kb.x[i] = 0;
+                kb.r[i] = r[c];
+                kb.q[i] = z[c];
+                kb.p[i] = z[c];
+            }
+        }
+        const float4 zf = make_float4((float)z[0], (float)z[1], (float)z[2], 0.f);
+        if (np.minres && kb.Zf[0]) {
+            reinterpret_cast<float4*>(kb.Zf[0])[n] = zf;
+            reinterpret_cast<float4*>(kb.Zf[1])[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (!np.minres && kb.pf) reinterpret_cast<float4*>(kb.pf)[n] = zf;
+    }
+    // the preconditioner is the mass: the Newton norm and z . r are one sum
+    acc = block_sum_fused(acc);
+    if (threadIdx.x == 0) na.part_norm[blockIdx.x] = acc;
+    if (!grid_sync(gs, epoch, limit, flags)) return false;
+    const double zr = reduce_partials_fused(na.part_norm, gridDim.x);
+    const double norm = sqrt(zr);
+    const bool done = (norm < np.tol) || !(norm == norm);
+    // MIXED: a norm that did not halve means FP32 stress round-off now
+    // dominates the residual; the rest of the solve evaluates it in FP64, and
+    // this iteration takes no step (the residual is re-evaluated first)
+    const bool stall = np.escalate && !done && !was_fp64 && nit > 0 && !(norm <= 0.5 * last);
+    const double mx = norm > np.tol ? norm : np.tol;
+    const double rel0 = np.tol_scale * sqrt(mx);
+    const double rel = rel0 < 0.5 ? rel0 : 0.5;
+    out.zr = zr;
+    out.rnorm = norm;
+    out.local_tol = fmin(rel * norm, np.abs_tol);
+    out.active = !done && !stall && !(norm < out.local_tol) && np.kmax > 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { // every CTA has read sc before the barrier
+        if (nit == 0) sc->res_initial = norm;
+        if (stall) sc->fp64_res = 1;
+        sc->res_final = norm;
+        sc->kit = 0;
+        sc->kactive = out.active ? 1 : 0;
+        if (done) {
+            sc->newton_done = 1;
+            sc->converged = (norm == norm) ? 1 : 0;
+        }
+        else {
+            sc->rel_tol = rel;
+            sc->rnorm = norm;
+            sc->local_tol = out.local_tol;
+        }
+    }
+    return true;
+}
+
+// End of a Newton iteration that solved: dv += x (with MINRES's deferred last
+// update), vstar = vn + dv on active nodes.  A thread's nodes are those whose
+// x, M and Z it wrote in the solve's node passes.
+template <int NPB>
+__device__ __forceinline__ void newton_step(NodeGeom ng, const NewtonArgs& na, const double* __restrict__ gm, const KrylovBufs& kb,
+    const MrPending& pd, bool minres)
+{
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t n = t0; n < ng.nn; n += nt) {
+        if (gm[n] == 0) continue; // vstar stays 0
+        double vs[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int64_t i = vidx<NPB>(n, c);
+            double step = !minres || pd.hasx ? kb.x[i] : 0.0; // MINRES: x exists from its second iteration on
+            if (pd.on) step += pd.t * mr_direction(pd, i);
+            const double d = na.dv[i] + step;
+            na.dv[i] = d;
+            vs[c] = na.vn[i] + d;
+            na.vstar[i] = vs[c];
+        }
+        if (na.vstar_f) na.vstar_f[n] = make_float4((float)vs[0], (float)vs[1], (float)vs[2], 0.f);
+    }
+}
+
+// NEWTON: a whole Newton iteration from its residual (newton_begin) to its step;
+// else the solve alone, started by other kernels (the adjoint).
+template <class L, class T, class TX, bool NEWTON>
+__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_persistent(NodeGeom ng, HvpArgs ha, NewtonArgs na, const double* __restrict__ gm,
     const int8_t* __restrict__ col, const double* __restrict__ P6, double dt2, KrylovBufs kb, double* __restrict__ part_a,
     double* __restrict__ part_b, SolverScalars* __restrict__ sc, int kmax, GridSync* __restrict__ gs, long long limit, int32_t* __restrict__ flags)
 {
-    if (sc->newton_done || !sc->kactive) return;
+    if (sc->newton_done || (!NEWTON && !sc->kactive)) return;
     constexpr int NPB = L::NPB;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     HvpSmem<L, T, TX>& hs = *reinterpret_cast<HvpSmem<L, T, TX>*>(smem_raw);
@@ -559,15 +598,26 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_p
     int phase = 0;
     unsigned epoch = 0;
     const int nit = sc->nit;
-    int k = sc->kit;
-    double zTr = sc->mr[k & 1][0];
+    int k = 0;
+    double zTr, local_tol;
+    if constexpr (NEWTON) {
+        SolveStart ss;
+        if (!newton_begin<NPB>(ng, na, gm, col, P6, kb, sc, gs, epoch, limit, flags, ss)) return;
+        if (!ss.active) return;
+        zTr = ss.zr;
+        local_tol = ss.local_tol;
+    }
+    else {
+        k = sc->kit;
+        zTr = sc->mr[k & 1][0];
+        local_tol = sc->local_tol;
+    }
     // the product's input: p, or its FP32 node-major copy when TX is float
     const TX* pin;
     if constexpr (sizeof(TX) == 4)
         pin = reinterpret_cast<const TX*>(kb.pf);
     else
         pin = reinterpret_cast<const TX*>(kb.p);
-    const double local_tol = sc->local_tol;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     for (;;) {
         // the Hessian-vector product of p into hacc
@@ -691,9 +741,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_p
             sc->kit = k;
             if (!go) sc->kactive = 0;
         }
-        if (!go) return;
+        if (!go) break;
         if (!grid_sync(gs, epoch, limit, flags)) return; // p complete before the next product
     }
+    if constexpr (NEWTON) newton_step<NPB>(ng, na, gm, kb, MrPending{}, false);
 }
 
 // ------------------------------------------------ persistent MINRES -----
@@ -712,25 +763,38 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_p
 // from it).  Three bounded grid barriers per iteration: the product is
 // complete before the operator pass reads hacc, W before the Lanczos step, and
 // Z~_{k+1} before the next product and the reduction of its norm.
-template <class L, class T, class TX, class Model>
-__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_mr_persistent(NodeGeom ng, HvpArgs ha, Model model, const double* __restrict__ gm,
+// NEWTON: a whole Newton iteration from its residual (newton_begin) to its step;
+// else the solve alone (ADMM).
+template <class L, class T, class TX, class Model, bool NEWTON>
+__global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_mr_persistent(NodeGeom ng, HvpArgs ha, NewtonArgs na, Model model, const double* __restrict__ gm,
     const int8_t* __restrict__ col, const double* __restrict__ P6, double dt2, KrylovBufs kb, double* __restrict__ part_a,
     double* __restrict__ part_b, SolverScalars* __restrict__ sc, int kmax, GridSync* __restrict__ gs, long long limit, int32_t* __restrict__ flags)
 {
-    if (sc->newton_done || !sc->kactive) return;
+    if (sc->newton_done || (!NEWTON && !sc->kactive)) return;
     constexpr int NPB = L::NPB;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     HvpSmem<L, T, TX>& hs = *reinterpret_cast<HvpSmem<L, T, TX>*>(smem_raw);
     __shared__ double mst[MST_N];
     double* const pend = mst + MST_PEND;
-    int k = sc->kit;
-    if (threadIdx.x == 0) mr_load(sc, mst, k);
+    int k = 0;
+    double local_tol;
+    unsigned epoch = 0;
+    const int nit = sc->nit;
+    if constexpr (NEWTON) {
+        SolveStart ss;
+        if (!newton_begin<NPB>(ng, na, gm, col, P6, kb, sc, gs, epoch, limit, flags, ss)) return;
+        if (!ss.active) return;
+        local_tol = ss.local_tol;
+        if (threadIdx.x == 0) mr_init(mst, ss.rnorm);
+    }
+    else {
+        k = sc->kit;
+        local_tol = sc->local_tol;
+        if (threadIdx.x == 0) mr_load(sc, mst, k);
+    }
     group_smem_init(hs);
     Share share(ha.ga);
     int phase = 0;
-    unsigned epoch = 0;
-    const int nit = sc->nit;
-    const double local_tol = sc->local_tol;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     for (;;) {
         // the product of Z~_k into hacc
@@ -804,37 +868,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_mr_p
         ++k;
         const bool go = !(rnorm < local_tol || k >= kmax);
         mr_store(sc, mst, k, nit, rnorm, go);
-        if (!go) return;
+        if (!go) break;
     }
-}
-
-// dv += x (the linear solve's step, with MINRES's deferred last update);
-// vstar = vn + dv on active nodes.
-template <int NPB>
-__global__ void __launch_bounds__(ND_THREADS) k_newton_step(NodeGeom ng, const double* __restrict__ gm, KrylovBufs kb, int minres,
-    const double* __restrict__ vn, double* __restrict__ dv, double* __restrict__ vstar, const SolverScalars* __restrict__ sc,
-    float4* __restrict__ vstar_f)
-{
-    if (sc->newton_done) return;
-    const MrPending pd = mr_pending(kb, sc->pend, minres ? sc->kit : 0);
-    for (int64_t n = (int64_t)blockIdx.x * ND_THREADS + threadIdx.x; n < ng.nn; n += (int64_t)gridDim.x * ND_THREADS) {
-        const bool act = gm[n] != 0;
-        double vs[3];
-        for (int k = 0; k < 3; ++k) {
-            int64_t i = vidx<NPB>(n, k);
-            double d = dv[i];
-            if (act) {
-                // MINRES: x exists from its second iteration on
-                double step = !minres || pd.hasx ? kb.x[i] : 0.0;
-                if (pd.on) step += pd.t * mr_direction(pd, i);
-                d += step;
-                dv[i] = d;
-            }
-            vs[k] = act ? vn[i] + d : 0.0;
-            vstar[i] = vs[k];
-        }
-        if (vstar_f) vstar_f[n] = make_float4((float)vs[0], (float)vs[1], (float)vs[2], 0.f);
-    }
+    if constexpr (NEWTON) newton_step<NPB>(ng, na, gm, kb, mr_pending(kb, pend, k), true);
 }
 
 // The FP32 node-major copy of vstar ([B][NPB][4]) that the MIXED particle
@@ -1174,31 +1210,19 @@ struct NewtonLaunch {
     int nb;
 };
 
-// First part of a Newton iteration: update, residual with the Krylov start
-// vectors, check and Krylov start.
-template <int NPB>
-int launch_newton_head(const NewtonLaunch& L, cudaStream_t st)
+NewtonArgs newton_args(const NewtonLaunch& L)
 {
     Ctx* ctx = L.ctx;
-    int rc = launch_update(ctx);
-    if (rc) return rc;
-    const double* g = ctx->cfg.gravity;
-    k_residual_start<NPB><<<L.nb, ND_THREADS, 0, st>>>(L.ng, ctx->gm.as<double>(), ctx->facc.as<double>(), ctx->dv.as<double>(),
-        ctx->collided.as<int8_t>(), ctx->proj.as<double>(), g[0], g[1], g[2], ctx->dt, L.kb, L.np.minres, L.pA, L.pB, L.sc);
-    k_newton_start<NPB><<<1, ND_THREADS, 0, st>>>(L.ng, L.np, L.pA, L.pB, L.sc);
-    g_kernel_launches += 2;
-    return ZMPM_OK;
-}
-
-template <int NPB>
-int launch_newton_tail(const NewtonLaunch& L, cudaStream_t st, cudaGraphConditionalHandle hN, int use_graph)
-{
-    Ctx* ctx = L.ctx;
-    k_newton_step<NPB><<<L.nb, ND_THREADS, 0, st>>>(L.ng, ctx->gm.as<double>(), L.kb, L.np.minres, ctx->vn.as<double>(), ctx->dv.as<double>(),
-        ctx->vstar.as<double>(), L.sc, ctx->mixed ? ctx->vstarf.as<float4>() : nullptr);
-    k_newton_advance<<<1, 1, 0, st>>>(L.sc, L.np.nmax, hN, use_graph, L.ctx->gsync.as<GridSync>());
-    g_kernel_launches += 2;
-    return ZMPM_OK;
+    NewtonArgs na = {};
+    na.np = L.np;
+    na.facc = ctx->facc.as<double>();
+    na.dv = ctx->dv.as<double>();
+    na.vn = ctx->vn.as<double>();
+    na.vstar = ctx->vstar.as<double>();
+    na.vstar_f = ctx->mixed ? ctx->vstarf.as<float4>() : nullptr;
+    na.part_norm = L.pB;
+    for (int d = 0; d < 3; ++d) na.g[d] = ctx->cfg.gravity[d];
+    return na;
 }
 
 // CTAs that a persistent solve can occupy: by its products or by two nodes per
@@ -1210,7 +1234,7 @@ int64_t useful_solve(const Ctx* ctx)
 }
 
 // The persistent CG solve (k_cg_persistent) on the Newton operator.
-template <int NPB>
+template <int NPB, bool NEWTON>
 int launch_cg_persistent(const NewtonLaunch& L, cudaStream_t st)
 {
     Ctx* ctx = L.ctx;
@@ -1226,10 +1250,10 @@ int launch_cg_persistent(const NewtonLaunch& L, cudaStream_t st)
             ctx->err = "MIXED CG needs the FP32 copy of p";
             return ZMPM_BAD_ARG;
         }
-        return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, float>), k_cg_persistent<Lay, float, float>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
+        return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, float>), k_cg_persistent<Lay, float, float, NEWTON>, L.ng, ha, newton_args(L), gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
             ctx->spin_limit, flags);
     }
-    return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_cg_persistent<Lay, double, double>, L.ng, ha, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
+    return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_cg_persistent<Lay, double, double, NEWTON>, L.ng, ha, newton_args(L), gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs,
         ctx->spin_limit, flags);
 }
 
@@ -1250,9 +1274,9 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
     const long long lim = ctx->spin_limit;
     if (admm) {
         if (ctx->mixed)
-            return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, double>), k_mr_persistent<Lay, float, double, AdmmOpModel<float>>, L.ng, ha,
+            return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, double>), k_mr_persistent<Lay, float, double, AdmmOpModel<float>, false>, L.ng, ha, newton_args(L),
                 AdmmOpModel<float>{ ctx->adm_B.as<float>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
-        return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_mr_persistent<Lay, double, double, AdmmOpModel<double>>, L.ng, ha,
+        return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_mr_persistent<Lay, double, double, AdmmOpModel<double>, false>, L.ng, ha, newton_args(L),
             AdmmOpModel<double>{ ctx->adm_B.as<double>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
     }
     if (ctx->mixed) {
@@ -1260,11 +1284,11 @@ int launch_mr_persistent(const NewtonLaunch& L, cudaStream_t st, bool admm)
             ctx->err = "MIXED MINRES needs the FP32 copies of Z";
             return ZMPM_BAD_ARG;
         }
-        return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, float>), k_mr_persistent<Lay, float, float, HvpModel<float>>, L.ng, ha,
+        return launch_resident(ctx, st, true, useful_solve<float>(ctx), sizeof(HvpSmem<Lay, float, float>), k_mr_persistent<Lay, float, float, HvpModel<float>, true>, L.ng, ha, newton_args(L),
             HvpModel<float>{ ha.pi, ctx->scratch.as<float>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim,
             flags);
     }
-    return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_mr_persistent<Lay, double, double, HvpModel<double>>, L.ng, ha,
+    return launch_resident(ctx, st, true, useful_solve<double>(ctx), sizeof(HvpSmem<Lay, double, double>), k_mr_persistent<Lay, double, double, HvpModel<double>, true>, L.ng, ha, newton_args(L),
         HvpModel<double>{ ha.pi, ctx->scratch.as<double>(), ctx->Pcap }, gm, col, P6, L.dt2, L.kb, L.pA, L.pC, L.sc, L.np.kmax, gs, lim, flags);
 }
 
@@ -1313,17 +1337,25 @@ int while_graph(Ctx* ctx, Body&& body, cudaGraphExec_t* exec_out)
     return ZMPM_OK;
 }
 
-// One Newton iteration with its linear solve as one persistent kernel
-// (k_mr_persistent or k_cg_persistent): update, residual and Krylov start,
-// Newton check, the solve, step and advance.
+// The linear solve of a Newton iteration with the iteration's residual, check
+// and step, as one persistent kernel (k_mr_persistent or k_cg_persistent).
+template <int NPB>
+int launch_newton_solve(const NewtonLaunch& L, cudaStream_t st)
+{
+    return L.np.minres ? launch_mr_persistent<NPB>(L, st, false) : launch_cg_persistent<NPB, true>(L, st);
+}
+// One Newton iteration: update, persistent solve, advance (a kernel of its own:
+// it runs, and ends the loop, whatever became of the solve's barriers).
 template <int NPB>
 int launch_newton_iteration(const NewtonLaunch& L, cudaStream_t st, cudaGraphConditionalHandle hN, int use_graph)
 {
-    int rc = launch_newton_head<NPB>(L, st);
+    int rc = launch_update(L.ctx);
     if (rc) return rc;
-    rc = L.np.minres ? launch_mr_persistent<NPB>(L, st, false) : launch_cg_persistent<NPB>(L, st);
+    rc = launch_newton_solve<NPB>(L, st);
     if (rc) return rc;
-    return launch_newton_tail<NPB>(L, st, hN, use_graph);
+    k_newton_advance<<<1, 1, 0, st>>>(L.sc, L.np.nmax, hN, use_graph, L.ctx->gsync.as<GridSync>());
+    ++g_kernel_launches;
+    return ZMPM_OK;
 }
 
 // The Newton solve as one graph: WHILE(Newton){ iteration }.
@@ -1414,14 +1446,14 @@ static int newton_impl(Ctx* ctx, const zmpm_solver& s)
         ctx->hvp_ev.push_back(e);
     }
     for (int it = 0; it < s.newton_max_iterations; ++it) {
-        int rc = launch_newton_head<NPB>(L, st);
+        int rc = launch_update(ctx);
         if (rc) return rc;
         ZMPM_CUDA(cudaEventRecord(ctx->hvp_ev[2 * it], st));
-        rc = L.np.minres ? launch_mr_persistent<NPB>(L, st, false) : launch_cg_persistent<NPB>(L, st);
+        rc = launch_newton_solve<NPB>(L, st);
         if (rc) return rc;
         ZMPM_CUDA(cudaEventRecord(ctx->hvp_ev[2 * it + 1], st));
-        rc = launch_newton_tail<NPB>(L, st, 0, 0);
-        if (rc) return rc;
+        k_newton_advance<<<1, 1, 0, st>>>(L.sc, L.np.nmax, 0, 0, ctx->gsync.as<GridSync>());
+        ++g_kernel_launches;
         ZMPM_CUDA(cudaGetLastError());
     }
     return ZMPM_OK;
@@ -1632,7 +1664,7 @@ int run_adjoint_solve(Ctx* ctx, double tol, int max_iterations)
     }
     g_kernel_launches += 2;
     ZMPM_CUDA(cudaMemsetAsync(ctx->gsync.p, 0, sizeof(GridSync), st));
-    int rc = ctx->layout == 1 ? launch_cg_persistent<32>(Lc, st) : launch_cg_persistent<64>(Lc, st);
+    int rc = ctx->layout == 1 ? launch_cg_persistent<32, false>(Lc, st) : launch_cg_persistent<64, false>(Lc, st);
     if (rc) return rc;
     ZMPM_CUDA(cudaStreamSynchronize(st));
     ZMPM_CUDA(cudaGetLastError());

@@ -2,9 +2,6 @@
 //
 // Kernels
 //  k_p2g_reg particlesToGridHelper<APIC> (MpmSimulationBase.cpp:563-608)
-//  k_stress  MpmForceBase::updatePositionBasedState (MpmForceBase.cpp:306-344):
-//            G2P of grad(vn+dv), F = (I + dt grad v) Fn, stress and Hessian scratch
-//            (the FP64 evaluation of a MIXED solve whose FP32 residual stalled)
 //  k_force   rasterizeForceToTVStack (MpmForceBase.cpp:102-152); also the
 //            explicit substep's and ADMM's force scatter
 //  k_update_fused  updatePositionBasedState + rasterizeForceToTVStack in one
@@ -265,87 +262,12 @@ int launch_damage(Ctx* ctx)
 }
 
 // --------------------------------------------------------------- update ----
-// Two kernels per Newton iteration (MpmForceBase::updatePositionBasedState then
-// rasterizeForceToTVStack, MpmForceBase.cpp:306-344, 102-152):
-//  k_stress: grad v at the particle from vstar = vn + dv, F = (I + dt grad v) Fn,
-//            S = V0 P(F) Fn^T (to `stress`) and the Hessian scratch; particles in
-//            slot order so every particle array is read coalesced.
-//  k_force : facc -= sum_p S_p grad w_ip, layered conflict-free scatter.
-// gate (MIXED contexts, which launch an FP32 and an FP64 pair of k_stress /
-// k_force per Newton iteration): 0 always runs, 1 runs while the solve's
-// residual is FP32, 2 once it is FP64.  frac_x: B-spline weights from the FP64
-// positions instead of the stored fractions (the FP64 residual of MIXED).
+// gate (MIXED contexts, which launch the FP32 and the FP64 form of
+// k_update_fused per Newton iteration): 0 always runs, 1 runs while the solve's
+// residual is FP32, 2 once it is FP64.
 __device__ __forceinline__ bool gated_off(const SolverScalars* sc, int gate)
 {
     return sc && (sc->newton_done || (gate != 0 && (gate == 1) == (sc->fp64_res != 0)));
-}
-
-template <class L, class TS, class TH>
-__global__ void __launch_bounds__(XF_THREADS) k_stress(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    const double* __restrict__ pd, const int32_t* __restrict__ pi, int64_t cap, const short4* __restrict__ base, double dx, double dt,
-    const TH* __restrict__ frac, const double* __restrict__ vstar, TS* __restrict__ stress, TH* __restrict__ scr,
-    const SolverScalars* __restrict__ sc, int32_t* __restrict__ flags, int gate, int frac_x)
-{
-    if (gated_off(sc, gate)) return;
-    constexpr int NPB = L::NPB;
-    __shared__ __align__(128) double win[8 * 3 * NPB];
-    __shared__ int32_t nbr[8];
-    __shared__ __align__(8) uint64_t bar;
-    const int g = blockIdx.x;
-    if (threadIdx.x < 8) nbr[threadIdx.x] = group_nbr[8 * g + threadIdx.x];
-    __syncthreads();
-    stage_window<NPB>(win, vstar, nbr, &bar, flags);
-    const TS inv_dx = TS(1.0 / dx);
-    const TS tdt = TS(dt);
-    const int s0 = group_start[g], s1 = group_start[g + 1];
-    for (int s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
-        const int kind = pi[PI_KIND * cap + s];
-        if (kind == ZMPM_MODEL_NONE) {
-#pragma unroll
-            for (int q = 0; q < 9; ++q) stress[q * cap + s] = TS(0);
-            continue;
-        }
-        const short4 b = base[s];
-        TS w[3][3], dwr[3][3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-            bspline(frac_x ? (TS)((1.0 / dx) * pd[(PD_X + d) * cap + s] - (double)((&b.x)[d])) : (TS)frac[d * cap + s], w[d], dwr[d]);
-        const int lx = b.x & (L::BX - 1), ly = b.y & (L::BY - 1), lz = b.z & (L::BZ - 1);
-        M3<TS> gv = m3_zero<TS>();
-        for_stencil<L>(lx, ly, lz, w, dwr, inv_dx, [&](int t, int e, int, int, int, TS, const TS* dw) {
-            const double* vv = win + t * 3 * NPB + e;
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                TS vr = (TS)vv[r * NPB];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) gv(r, c) += vr * dw[c];
-            }
-        });
-        M3<TS> Fn, A = m3_identity<TS>();
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            Fn.a[q] = (TS)pd[(PD_F + q) * cap + s];
-            A.a[q] += tdt * gv.a[q];
-        }
-        M3<TS> F = m3_mul(A, Fn);
-        ModelParams mp{ pd[PD_MU * cap + s], pd[PD_LAM * cap + s], pd[PD_KAPPA * cap + s], pd[PD_G * cap + s] };
-        const double V0 = pd[PD_VOL * cap + s];
-        bool degenerate = false;
-        M3<TS> S = model_update<TS, TH>(kind, mp, (TS)V0, F, Fn, scr, cap, s, sizeof(TS) == 4 ? &degenerate : nullptr);
-        if constexpr (sizeof(TS) == 4) {
-            if (degenerate) { // FP64 re-evaluation of near-degenerate particles
-                M3<double> Fnd, Ad = m3_identity<double>();
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    Fnd.a[q] = pd[(PD_F + q) * cap + s];
-                    Ad.a[q] += dt * (double)gv.a[q];
-                }
-                S = m3_cast<TS>(model_update<double, TH>(kind, mp, V0, m3_mul(Ad, Fnd), Fnd, scr, cap, s, nullptr));
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) stress[q * cap + s] = S.a[q];
-    }
 }
 
 // Explicit substep: FBasedMpmForceHelper::updateState (FBasedMpmForceHelper.cpp:
@@ -514,25 +436,31 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_prod
 // the restored Fn, FBasedMpmForceHelper.cpp:95-109), S = V0 P(F) Fn^T and the
 // Hessian scratch (updateImplicitState, :68-92); FP32 evaluations of
 // near-degenerate SVDs are redone in FP64.  Phase 2 adds -S_p grad w_ip to
-// facc.  gate as k_stress / k_force.
-template <class L, class T, class TX>
+// facc.  TH: the type of the stored fractions and the scratch; T = double with TH
+// = float is the FP64 residual of a MIXED solve (weights from the positions).
+template <class L, class T, class TX, class TH>
 struct UpdatePhase1 {
     const double* pd;
     const int32_t* pi;
     int64_t cap;
     const short4* base;
-    const T* frac;
-    T* scr;
+    const TH* frac;
+    TH* scr;
     unsigned long long* svd64;
     double inv_dx, dt;
 
     template <int FS>
     __device__ __forceinline__ void run(const TX* win, int64_t s, T* rc) const
     {
+        const short4 b = base[s];
         T fr[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) fr[d] = frac[d * cap + s];
-        const short4 b = base[s];
+        for (int d = 0; d < 3; ++d) {
+            if constexpr (sizeof(T) == sizeof(TH))
+                fr[d] = frac[d * cap + s];
+            else
+                fr[d] = inv_dx * pd[(PD_X + d) * cap + s] - (double)((&b.x)[d]);
+        }
         const int kind = pi[PI_KIND * cap + s];
 #pragma unroll
         for (int d = 0; d < 3; ++d) rc[d * FS] = fr[d];
@@ -557,7 +485,7 @@ struct UpdatePhase1 {
             const ModelParams mp{ pd[PD_MU * cap + s], pd[PD_LAM * cap + s], pd[PD_KAPPA * cap + s], pd[PD_G * cap + s] };
             const double V0 = pd[PD_VOL * cap + s];
             bool degenerate = false;
-            S = model_update<T, T>(kind, mp, (T)V0, m3_mul(A, Fn), Fn, scr, cap, s, sizeof(T) == 4 ? &degenerate : nullptr);
+            S = model_update<T, TH>(kind, mp, (T)V0, m3_mul(A, Fn), Fn, scr, cap, s, sizeof(T) == 4 ? &degenerate : nullptr);
             if constexpr (sizeof(T) == 4) {
                 if (degenerate) { // FP64 re-evaluation of near-degenerate particles
                     atomicAdd(svd64, 1ull);
@@ -579,10 +507,10 @@ struct UpdatePhase1 {
 };
 constexpr int UPDATE_PIECE = 64; // fixed cost of a piece in particles
 
-template <class L, class T, class TX>
+template <class L, class T, class TX, class TH>
 __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_update_fused(GroupArgs ga, const double* __restrict__ pd,
-    const int32_t* __restrict__ pi, int64_t cap, const short4* __restrict__ base, double dx, double dt, const T* __restrict__ frac,
-    const TX* __restrict__ vstar, T* __restrict__ scr, double* __restrict__ facc, const SolverScalars* __restrict__ sc,
+    const int32_t* __restrict__ pi, int64_t cap, const short4* __restrict__ base, double dx, double dt, const TH* __restrict__ frac,
+    const TX* __restrict__ vstar, TH* __restrict__ scr, double* __restrict__ facc, const SolverScalars* __restrict__ sc,
     int32_t* __restrict__ flags, int gate, unsigned long long* __restrict__ svd64)
 {
     if (gated_off(sc, gate)) return;
@@ -592,7 +520,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_upda
     Share share(ga);
     int ph = 0;
     group_share<L, T, TX, RowsScatter<T>, 3>(sm, ga, share, vstar, facc, nullptr, flags, ph,
-        UpdatePhase1<L, T, TX>{ pd, pi, cap, base, frac, scr, svd64, 1.0 / dx, dt });
+        UpdatePhase1<L, T, TX, TH>{ pd, pi, cap, base, frac, scr, svd64, 1.0 / dx, dt });
 }
 
 // ------------------------------------------------------------------ G2P ----
@@ -825,7 +753,7 @@ static int update_impl(Ctx* ctx, bool gated)
     DevCounters* dc = ctx->counters.as<DevCounters>();
     const SolverScalars* sc = gated ? ctx->scal.as<SolverScalars>() : nullptr;
     if (ctx->mixed) {
-        // FP32 stress and force; inside a solve also the FP64 pair, which runs
+        // FP32 stress and force; inside a solve also the FP64 form, which runs
         // instead once the FP32 residual stalled (FP32 Hessian scratch either
         // way).  The FP32 pass gathers from the FP32 copy of vstar, which the
         // Newton solve keeps current; the hooks and the adjoint set vstar directly.
@@ -836,25 +764,19 @@ static int update_impl(Ctx* ctx, bool gated)
             ctx->vstarf_valid = true;
         }
         int rc = launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, UPDATE_PIECE), sizeof(HvpSmem<L, float, float>),
-            k_update_fused<L, float, float>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(),
+            k_update_fused<L, float, float, float>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(),
             ctx->cfg.dx, ctx->dt, ctx->frac.as<float>(), ctx->vstarf.as<float>(), ctx->scratch.as<float>(), ctx->facc.as<double>(), sc, &dc->flags,
             gate, reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
         if (rc) return rc;
-        if (sc) {
-            k_stress<L, double, float><<<(unsigned)G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(),
-                ctx->group_nbr.as<int32_t>(), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx,
-                ctx->dt, ctx->frac.as<float>(), ctx->vstar.as<double>(), ctx->stress.as<double>(), ctx->scratch.as<float>(), sc, &dc->flags, 2,
-                1);
-            ++g_kernel_launches;
-            k_force<L, double, float><<<(unsigned)G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(),
-                ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<float>(), ctx->stress.as<double>(), ctx->facc.as<double>(), sc, 2,
-                ctx->pd.as<double>() + PD_X * ctx->Pcap);
-            ++g_kernel_launches;
-        }
+        if (sc)
+            return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, UPDATE_PIECE), sizeof(HvpSmem<L, double, double>),
+                k_update_fused<L, double, double, float>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap,
+                ctx->base.as<short4>(), ctx->cfg.dx, ctx->dt, ctx->frac.as<float>(), ctx->vstar.as<double>(), ctx->scratch.as<float>(),
+                ctx->facc.as<double>(), sc, &dc->flags, 2, reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
     }
     else {
         return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, UPDATE_PIECE), sizeof(HvpSmem<L, double, double>),
-            k_update_fused<L, double, double>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(),
+            k_update_fused<L, double, double, double>, group_args(ctx, UPDATE_PIECE), ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, ctx->base.as<short4>(),
             ctx->cfg.dx, ctx->dt, ctx->frac.as<double>(), ctx->vstar.as<double>(), ctx->scratch.as<double>(), ctx->facc.as<double>(), sc,
             &dc->flags, 0, reinterpret_cast<unsigned long long*>(&dc->svd_fp64));
     }
