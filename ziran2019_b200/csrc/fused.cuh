@@ -300,8 +300,15 @@ struct Share {
 // being flushed, the running one, the arriving one), and per warp the records
 // of its current chunk of particles, NF arrays of CH values (particle-minor:
 // phase 1's threads write consecutive words).  TX: the input window's type, or
-// void for kernels without one.  CH: what is left of the shared memory that lets
-// CTAS of these run on an SM (227 KB, 1 KB of it reserved per CTA).
+// void for kernels without one.  The accumulators are FP64 for FP32 arithmetic
+// too: the warps add in whatever order they get there, and FP32 sums in a varying
+// order moved a MIXED solve's residual by 10% at its FP32 floor from run to run,
+// and Newton iteration counts with it (an item's own FP32 sum has a fixed order).
+// FP32 kernels have one accumulator, FP64 kernels two: two FP64 ones, or an FP32
+// one per warp, left FP32 chunks of 74 particles, little more than half a warp's
+// usual share (1M particles: 3.69 and 3.60 ms per substep).
+// CH: what is left of the shared memory that lets CTAS of these run on an SM
+// (227 KB, 1 KB of it reserved per CTA).
 template <class L, class TX>
 struct InputWindow {
     static constexpr int ELEMS = VecWindow<L::NPB, TX>::ELEMS;
@@ -321,7 +328,8 @@ constexpr int FUSED_WARPS = FUSED_THREADS / 32;
 template <class L, class T, class TX, int NF, int NC>
 struct GroupSmem {
     using W = InputWindow<L, TX>;
-    static constexpr size_t FIXED = 2 * (W::ELEMS * sizeof(typename W::Elem) + 8 * NC * L::NPB * sizeof(T)) + 3 * sizeof(MetaBuf<L>) + 512;
+    static constexpr int ACCS = sizeof(T) == 4 ? 1 : 2;
+    static constexpr size_t FIXED = 2 * W::ELEMS * sizeof(typename W::Elem) + ACCS * 8 * NC * L::NPB * sizeof(double) + 3 * sizeof(MetaBuf<L>) + 512;
     static constexpr size_t PER4 = 232448 / 4 - 1024, PER3 = 232448 / 3 - 1024;
     // four CTAs per SM where the windows leave room for records of a warp's usual share of a page, else three
     static constexpr int CTAS = FIXED + FUSED_WARPS * NF * 49 * sizeof(T) <= PER4 ? 4 : 3;
@@ -330,7 +338,7 @@ struct GroupSmem {
     static constexpr int FS = CH + 1; // odd: the fields of one particle fall in different banks
     static_assert(CH >= 32, "a chunk holds at least one particle per lane");
     alignas(128) typename W::Elem win[2][W::ELEMS ? W::ELEMS : 4];
-    alignas(16) T acc[2][8 * NC * L::NPB];
+    alignas(16) double acc[ACCS][8 * NC * L::NPB];
     alignas(16) MetaBuf<L> meta[3];
     alignas(8) uint64_t bar[2];
     alignas(16) T rec[FUSED_WARPS][NF * FS];
@@ -449,19 +457,21 @@ struct RowsScatter {
     }
 };
 
-// APIC P2G (particlesToGridHelper, MpmSimulationBase.cpp:563-608): item
-// (component r, cell) adds w_ip m_p (r = 0) or w_ip (q + a i + b j + c k)
-// (r >= 1, the momentum m (v + C (x_i - x_p)) written affinely in the node
-// offset (i, j, k)).  Records: fractions at 0-2, the mass at 3, (q, a, b, c) of
-// momentum component r - 1 at 4 r .. 4 r + 3.
-template <class T>
-struct P2gScatter {
-    static constexpr int NF = 16, NC = 4;
+// Affine: item (component, cell) adds w_ip (q + a i + b j + c k), a vector
+// written affinely in the node offset (i, j, k).  MASS (APIC P2G,
+// particlesToGridHelper, MpmSimulationBase.cpp:563-608): component 0 adds w_ip
+// m_p and components 1-3 the momentum m (v + C (x_i - x_p)); without it the
+// three components are a vector (the MLS-MPM force).  Records: fractions at
+// 0-2, the mass at 3 if any, then (q, a, b, c) of each vector component.
+template <class T, bool MASS>
+struct AffineScatter {
+    static constexpr int NF = MASS ? 16 : 15, NC = MASS ? 4 : 3;
     template <int FS>
     __device__ __forceinline__ static void sum(const T* rec, int r, int p0, int p1, int part, int parts, T a[27])
     {
         const T* fr = rec;
-        const T* row = rec + (r == 0 ? 3 : 4 * r) * FS;
+        const bool vec = !MASS || r != 0;
+        const T* row = rec + (MASS ? (vec ? 4 * r : 3) : 3 + 4 * r) * FS;
         if constexpr (sizeof(T) == 4) {
             float2 a2[27];
 #pragma unroll
@@ -474,7 +484,7 @@ struct P2gScatter {
                 for (int d = 0; d < 3; ++d) bspline_all2(f2(fr[d * FS + p], fr[d * FS + pq]), w[d], dw[d]);
                 const float2 q0 = f2(row[p], sq * row[pq]);
                 float2 ax = f2(0.f), by = f2(0.f), cz = f2(0.f);
-                if (r != 0) {
+                if (vec) {
                     ax = f2(row[FS + p], sq * row[FS + pq]);
                     by = f2(row[2 * FS + p], sq * row[2 * FS + pq]);
                     cz = f2(row[3 * FS + p], sq * row[3 * FS + pq]);
@@ -506,7 +516,7 @@ struct P2gScatter {
 #pragma unroll
                 for (int d = 0; d < 3; ++d) bspline_all(fr[d * FS + p], w[d], dw[d]);
                 const T q0 = row[p];
-                const T ax = r ? row[FS + p] : T(0), by = r ? row[2 * FS + p] : T(0), cz = r ? row[3 * FS + p] : T(0);
+                const T ax = vec ? row[FS + p] : T(0), by = vec ? row[2 * FS + p] : T(0), cz = vec ? row[3 * FS + p] : T(0);
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
 #pragma unroll
@@ -556,7 +566,7 @@ __device__ __forceinline__ void group_warp(GroupSmem<L, T, TX, Scatter::NF, Scat
     const int b0 = st[occ[lo]], e1 = st[occ[hi - 1] + 1];
     const int p_lo = b0 > a0 ? b0 : a0, p_hi = e1 < a1 ? e1 : a1;
     T* rec = sm.rec[warp];
-    T* acc = sm.acc[ph & 1];
+    double* acc = sm.acc[SM::ACCS == 2 ? ph & 1 : 0];
     const int ncell = hi - lo, items = NC * ncell;
     for (int c0 = p_lo; c0 < p_hi; c0 += SM::CH) {
         const int c1 = c0 + SM::CH < p_hi ? c0 + SM::CH : p_hi;
@@ -580,24 +590,26 @@ __device__ __forceinline__ void group_warp(GroupSmem<L, T, TX, Scatter::NF, Scat
 #pragma unroll
                 for (int m = 0; m < 27; ++m) a[m] += __shfl_down_sync(0xffffffffu, a[m], width);
             }
-            if (p0 >= p1 || part) continue;
+            const bool add = p0 < p1 && !part;
             const int lx = ce >> (L::YB + L::ZB), ly = (ce >> L::ZB) & (L::BY - 1), lz = ce & (L::BZ - 1);
             const StencilOffsets<L> so(lx, ly, lz);
+            if (!add) continue;
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) atomicAdd(acc + window_scalar<NPB>(so.X[i] + so.Y[j] + so.Z[k], r, NC), a[9 * i + 3 * j + k]);
+                    for (int k = 0; k < 3; ++k)
+                        atomicAdd(acc + window_scalar<NPB>(so.X[i] + so.Y[j] + so.Z[k], r, NC), (double)a[9 * i + 3 * j + k]);
         }
     }
 }
 
 // All pieces of the CTA's share: out += the scattered sums (component c < NC0
 // to outa [B][NC0][NPB], the rest to outb).  All threads call it; ph counts the
-// CTA's pieces over the kernel.  One block barrier per piece: it separates the
-// piece's sums from their flush, and the flush (which leaves its buffer zero)
-// from the buffer's next use two pieces later.
+// CTA's pieces over the kernel.  A block barrier separates a piece's sums from
+// their flush, which leaves its accumulators zero; FP32 has a second one before
+// their next use, FP64 uses the other buffer meanwhile.
 template <class L, class T, class TX, class Scatter, int NC0, class Phase1>
 __device__ __forceinline__ void group_share(GroupSmem<L, T, TX, Scatter::NF, Scatter::NC>& sm, const GroupArgs& a, Share& share, const TX* x,
     double* __restrict__ outa, double* __restrict__ outb, int32_t* flags, int& ph, const Phase1& phase1)
@@ -617,19 +629,21 @@ __device__ __forceinline__ void group_share(GroupSmem<L, T, TX, Scatter::NF, Sca
         group_warp<L, T, TX, Scatter>(sm, cur, ph, phase1);
         cp_async_wait_all();
         __syncthreads();
-        T* acc = sm.acc[ph & 1];
+        using SM = GroupSmem<L, T, TX, Scatter::NF, Scatter::NC>;
+        double* acc = sm.acc[SM::ACCS == 2 ? ph & 1 : 0];
         const int32_t* nbr = sm.meta[ph % 3].nbr;
         for (int i = threadIdx.x; i < 8 * NC * NPB; i += FUSED_THREADS) {
-            const T v = acc[i];
-            if (v == T(0)) continue;
-            acc[i] = T(0);
+            const double v = acc[i];
+            if (v == 0) continue;
+            acc[i] = 0;
             const int t = i / (NC * NPB), r = i - t * NC * NPB, c = r / NPB, e = r - c * NPB;
             const int64_t blk = nbr[t];
             if (c < NC0)
-                atomicAdd(&outa[(blk * NC0 + c) * NPB + e], (double)v);
+                atomicAdd(&outa[(blk * NC0 + c) * NPB + e], v);
             else
-                atomicAdd(&outb[(blk * (NC - NC0) + (c - NC0)) * NPB + e], (double)v);
+                atomicAdd(&outb[(blk * (NC - NC0) + (c - NC0)) * NPB + e], v);
         }
+        if constexpr (SM::ACCS == 1) __syncthreads(); // the accumulator is clear
         cur = nxt;
         have = more;
         ++ph;

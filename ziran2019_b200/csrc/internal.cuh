@@ -256,7 +256,7 @@ int upload(Ctx* ctx);      // host scene arrays -> device pools (once per edit)
 int download(Ctx* ctx);    // device pools -> host scene arrays (particle order)
 int begin_edit(Ctx* ctx);  // download, then mark the device copy stale
 int run_explicit(Ctx* ctx, const zmpm_solver& s);      // symplectic substep up to G2P
-int launch_explicit_stress(Ctx* ctx);
+int launch_explicit_force(Ctx* ctx, double* out, bool mls); // out -= the explicit substep's forces (stress and scatter)
 int run_phase_field(Ctx* ctx, int32_t* iterations, double* residual); // FractureSimulation::solvePhaseFieldSystem after P2G
 int launch_phase_field_delete(Ctx* ctx);                               // FractureSimulation::deleteParticles before binning                  // V0 tau(F) (+ V0 tau(Fe)) into the stress buffer
 int launch_update(Ctx* ctx, bool gated = true);       // G2P(vn+dv) -> stress -> force P2G
@@ -276,7 +276,7 @@ int launch_admm_local(Ctx* ctx, double rho, double local_tol); // F step + rhs s
 int launch_admm_op(Ctx* ctx, const double* x, double* out); // out += sum (grad x B) grad w
 int launch_admm_dual(Ctx* ctx, double rho);            // y += rho omega (F - (I + dt grad v) Fn)
 int launch_admm_lastdv(Ctx* ctx);                      // last_dv = sum dv w / (dt sum w)
-int launch_force_scatter(Ctx* ctx, double* out, bool mls = false);       // out -= sum_p stress_p grad w_ip (stress buffer)
+int launch_force_scatter(Ctx* ctx, double* out);       // out -= sum_p stress_p grad w_ip (stress buffer)
 int finalize_multiply(Ctx* ctx, const double* x, double* q); // q = project(m x + q)
 int ensure_node_buffers(Ctx* ctx);
 int compute_node_indices(Ctx* ctx);                    // getNumNodes numbering (hooks)

@@ -351,7 +351,7 @@ int launch_resident(Ctx* ctx, cudaStream_t st, bool coop, int64_t useful, size_t
 
 // CTAs that a pass over the particles in pieces can occupy: about PIECE_MIN
 // particles' worth of work each.
-constexpr int PIECE_MIN = 64;
+constexpr int PIECE_MIN = 32;
 inline int64_t useful_ctas(const Ctx* ctx, int K) { return (ctx->P + (int64_t)K * ctx->G + PIECE_MIN - 1) / PIECE_MIN; }
 
 } // namespace zmpm

@@ -1128,11 +1128,9 @@ int run_explicit(Ctx* ctx, const zmpm_solver& s)
     ZMPM_CUDA(cudaMemsetAsync(ctx->gm.p, 0, nn * sizeof(double), st));
     ZMPM_CUDA(cudaMemsetAsync(ctx->gmv.p, 0, 3 * nn * sizeof(double), st));
     ZMPM_CUDA(cudaMemsetAsync(ctx->facc.p, 0, 3 * nn * sizeof(double), st));
-    rc = launch_explicit_stress(ctx);
-    if (rc) return rc;
     rc = launch_p2g(ctx);
     if (rc) return rc;
-    rc = launch_force_scatter(ctx, ctx->facc.as<double>(), s.mls_mpm != 0);
+    rc = launch_explicit_force(ctx, ctx->facc.as<double>(), s.mls_mpm != 0);
     if (rc) return rc;
     rc = launch_damage(ctx);
     if (rc) return rc;

@@ -1,9 +1,10 @@
 // Particle <-> grid transfers of the implicit substep (helpers in xfer.cuh).
 //
 // Kernels
-//  k_p2g_reg particlesToGridHelper<APIC> (MpmSimulationBase.cpp:563-608)
-//  k_force   rasterizeForceToTVStack (MpmForceBase.cpp:102-152); also the
-//            explicit substep's and ADMM's force scatter
+//  k_p2g_fused particlesToGridHelper<APIC> (MpmSimulationBase.cpp:563-608)
+//  k_force   rasterizeForceToTVStack (MpmForceBase.cpp:102-152) of ADMM's
+//            right-hand side
+//  k_force_fused  the explicit substep's stress and force scatter
 //  k_update_fused  updatePositionBasedState + rasterizeForceToTVStack in one
 //            pass (gather of grad v, F, stress and Hessian scratch, force scatter)
 //  k_product  MpmForceBase::addScaledForceDifferential (MpmForceBase.cpp:259-302):
@@ -21,111 +22,9 @@
 namespace zmpm {
 
 // ------------------------------------------------------------------ P2G ----
-// Also writes each particle's fractional cell offsets (frac) for the FP32 HVP.
-// P2G with per-cell register accumulation: thread -> one cell of the page and
-// every (blockDim/NPB)-th particle of it; NCP of the four grid components
-// (mass, momentum x, y, z) are summed for the cell's 27 stencil nodes in
-// registers per pass and added to the shared window once per pass, so the
-// window sees one atomic per (thread, node, component) instead of one per
-// (particle, node, component).  APIC P2G: m_i += w m_p, (mv)_i += w m_p (v_p +
-// C_p (x_i - x_p)), in FP64 or, in MIXED contexts, FP32 (the grid sums are
-// FP64 in global memory either way).
-template <class L, class TH, int NCP>
-__global__ void __launch_bounds__(XF_THREADS, 3) k_p2g_reg(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    const double* __restrict__ pd, int64_t cap, const short4* __restrict__ base, double dx, double* __restrict__ gm, double* __restrict__ gmv,
-    TH* __restrict__ frac)
-{
-    using TA = TH; // arithmetic: FP64, or FP32 in MIXED contexts (the stored fractions' type)
-    constexpr int NPB = L::NPB;
-    __shared__ __align__(16) TA acc[8 * 4 * NPB];
-    __shared__ int32_t nbr[8];
-    __shared__ CellLayout<L> cl;
-    const int g = blockIdx.x;
-    if (threadIdx.x < 8) nbr[threadIdx.x] = group_nbr[8 * g + threadIdx.x];
-    zero_window<4, NPB>(acc);
-    const double inv_dx = 1.0 / dx;
-    const int s0 = group_start[g], s1 = group_start[g + 1];
-    build_cell_layout<L>(cl, base, s0, s1);
-    const int ce = threadIdx.x % NPB;
-    const int lx = ce >> (L::YB + L::ZB), ly = (ce >> L::ZB) & (L::BY - 1), lz = ce & (L::BZ - 1);
-    const int cnt = cl.cnt[ce], first = s0 + cl.start[ce];
-    const TA tdx = TA(dx);
-#pragma unroll 1
-    for (int c0 = 0; c0 < 4; c0 += NCP) {
-        TA a[27][NCP];
-#pragma unroll
-        for (int n = 0; n < 27; ++n)
-#pragma unroll
-            for (int c = 0; c < NCP; ++c) a[n][c] = TA(0);
-        for (int r = threadIdx.x / NPB; r < cnt; r += blockDim.x / NPB) {
-            const int s = first + r;
-            const short4 b = base[s];
-            double xp[3];
-            TA fr[3], w[3][3], dwr[3][3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                xp[d] = pd[(PD_X + d) * cap + s];
-                const double d0 = inv_dx * xp[d] - (double)((&b.x)[d]);
-                if (c0 == 0) frac[d * cap + s] = (TH)d0;
-                fr[d] = (TA)d0;
-                bspline(fr[d], w[d], dwr[d]);
-            }
-            const double mass = pd[PD_M * cap + s];
-            TA mom[NCP], Cm[NCP][3];
-#pragma unroll
-            for (int c = 0; c < NCP; ++c) {
-                const int comp = c0 + c; // 0: mass, 1..3: momentum row comp-1
-                if (comp == 0) {
-                    mom[c] = (TA)mass;
-                    Cm[c][0] = Cm[c][1] = Cm[c][2] = TA(0);
-                }
-                else {
-                    const int rr = comp - 1;
-                    mom[c] = (TA)(mass * pd[(PD_V + rr) * cap + s]);
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) Cm[c][q] = (TA)(mass * pd[(PD_C + 3 * rr + q) * cap + s]);
-                }
-            }
-            for_stencil<L>(lx, ly, lz, w, dwr, TA(inv_dx), [&](int, int, int i, int j, int k, TA wijk, const TA*) {
-                // x_i - x_p: FP64 from the positions, FP32 from the cell fractions
-                TA xi[3];
-                if constexpr (sizeof(TA) == 8) {
-                    xi[0] = (b.x + i) * dx - xp[0];
-                    xi[1] = (b.y + j) * dx - xp[1];
-                    xi[2] = (b.z + k) * dx - xp[2];
-                }
-                else {
-                    xi[0] = (TA(i) - fr[0]) * tdx;
-                    xi[1] = (TA(j) - fr[1]) * tdx;
-                    xi[2] = (TA(k) - fr[2]) * tdx;
-                }
-                const int n = 9 * i + 3 * j + k;
-#pragma unroll
-                for (int c = 0; c < NCP; ++c) a[n][c] += (Cm[c][0] * xi[0] + Cm[c][1] * xi[1] + Cm[c][2] * xi[2] + mom[c]) * wijk;
-            });
-        }
-        if (threadIdx.x / NPB < cnt) {
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        int e;
-                        const int t = win_slot<L>(lx + i, ly + j, lz + k, e);
-                        TA* dst = acc + t * 4 * NPB + e;
-#pragma unroll
-                        for (int c = 0; c < NCP; ++c) atomicAdd(dst + (c0 + c) * NPB, a[9 * i + 3 * j + k][c]);
-                    }
-        }
-    }
-    __syncthreads();
-    flush_window<4, 1, NPB>(acc, nbr, gm, gmv);
-}
-
 // APIC P2G as a fused kernel (fused.cuh): phase 1 writes each particle's cell
 // fractions (also to `frac`, for the Newton kernels), its mass and the affine
-// form of its momentum; phase 2 (P2gScatter) sums them into the window by
+// form of its momentum; phase 2 (AffineScatter) sums them into the window by
 // (component, occupied cell) items.  T: arithmetic (FP32 in MIXED contexts);
 // the window is flushed into the FP64 grid sums.
 template <class L, class T>
@@ -164,7 +63,7 @@ struct P2gPhase1 {
     }
 };
 template <class L, class T>
-using P2gSmem = GroupSmem<L, T, void, P2gScatter<T>::NF, P2gScatter<T>::NC>;
+using P2gSmem = GroupSmem<L, T, void, AffineScatter<T, true>::NF, AffineScatter<T, true>::NC>;
 constexpr int P2G_PIECE = 96; // fixed cost of a piece in particles
 
 template <class L, class T>
@@ -176,7 +75,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, P2gSmem<L, T>::CTAS) k_p2g_fuse
     group_smem_init(sm);
     Share share(ga);
     int ph = 0;
-    group_share<L, T, void, P2gScatter<T>, 1>(sm, ga, share, nullptr, gm, gmv, flags, ph,
+    group_share<L, T, void, AffineScatter<T, true>, 1>(sm, ga, share, nullptr, gm, gmv, flags, ph,
         P2gPhase1<L, T>{ pd, cap, base, 1.0 / dx, T(dx), frac });
 }
 
@@ -270,72 +169,44 @@ __device__ __forceinline__ bool gated_off(const SolverScalars* sc, int gate)
     return sc && (sc->newton_done || (gate != 0 && (gate == 1) == (sc->fp64_res != 0)));
 }
 
-// Explicit substep: FBasedMpmForceHelper::updateState (FBasedMpmForceHelper.cpp:
-// 44-64) stores V0 tau(F) = V0 P(F) F^T per particle (slot order), plus V0
-// tau(Fe) for viscoelastic particles (FElasticNonequilibratedBasedMpmForceHelper.h:
-// 39-60).  TS precision with the FP64 re-evaluation of near-degenerate SVDs.
-template <class TS, class TH>
-__global__ void __launch_bounds__(XF_THREADS) k_explicit_stress(const double* __restrict__ pd, const int32_t* __restrict__ pi, int64_t cap,
-    int64_t P, TS* __restrict__ stress, TH* __restrict__ scr)
+// Force scatters: facc -= sum_p S_p grad w_ip (rasterizeForceToTVStack,
+// MpmForceBase.cpp:102-152), or with MLS the MLS-MPM weight of
+// particlesToGridWithForceHelper (MpmSimulationBase.cpp:527-541), facc -= (S_p
+// (x_i - x_p)) w_ip D^-1 with D^-1 = 4 / dx^2.  A particle's record from its S.
+template <class T, bool MLS, int FS>
+__device__ __forceinline__ void force_record(const M3<T>& S, const T fr[3], T inv_dx, T* rc)
 {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= P) return;
-    const int kind = pi[PI_KIND * cap + s];
-    M3<TS> S = m3_zero<TS>();
-    if (kind != ZMPM_MODEL_NONE) {
-        M3<TS> F;
 #pragma unroll
-        for (int q = 0; q < 9; ++q) F.a[q] = (TS)pd[(PD_F + q) * cap + s];
-        const ModelParams mp{ pd[PD_MU * cap + s], pd[PD_LAM * cap + s], pd[PD_KAPPA * cap + s], pd[PD_G * cap + s] };
-        const double V0 = pd[PD_VOL * cap + s];
-        bool degenerate = false;
-        S = model_update<TS, TH>(kind, mp, (TS)V0, F, F, scr, cap, s, sizeof(TS) == 4 ? &degenerate : nullptr);
-        if constexpr (sizeof(TS) == 4) {
-            if (degenerate) {
-                M3<double> Fd;
+    for (int d = 0; d < 3; ++d) rc[d * FS] = fr[d];
+    if constexpr (MLS) {
+        const T k = T(-4) * inv_dx; // dx D^-1
 #pragma unroll
-                for (int q = 0; q < 9; ++q) Fd.a[q] = pd[(PD_F + q) * cap + s];
-                S = m3_cast<TS>(model_update<double, TH>(kind, mp, V0, Fd, Fd, scr, cap, s, nullptr));
-            }
-        }
-        if (pi[PI_VISCO * cap + s]) {
-            M3<double> Fe;
+        for (int r = 0; r < 3; ++r) {
+            rc[(3 + 4 * r) * FS] = -k * (S(r, 0) * fr[0] + S(r, 1) * fr[1] + S(r, 2) * fr[2]);
 #pragma unroll
-            for (int q = 0; q < 9; ++q) Fe.a[q] = pd[(PD_FE + q) * cap + s];
-            const ModelParams mv{ pd[PD_VMU * cap + s], pd[PD_VLAM * cap + s], 0.0, 1.0 };
-            const M3<double> Se = model_update<double, TH>(ZMPM_MODEL_STVK_HENCKY_ISOTROPIC, mv, V0, Fe, Fe, scr, cap, s, nullptr);
-#pragma unroll
-            for (int q = 0; q < 9; ++q) S.a[q] += (TS)Se.a[q];
+            for (int c = 0; c < 3; ++c) rc[(4 + 4 * r + c) * FS] = k * S(r, c);
         }
     }
+    else {
 #pragma unroll
-    for (int q = 0; q < 9; ++q) stress[q * cap + s] = S.a[q];
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) rc[(3 + 3 * r + c) * FS] = -S(r, c) * inv_dx;
+    }
 }
 
-int launch_explicit_stress(Ctx* ctx)
-{
-    const int64_t P = ctx->P;
-    if (P == 0) return ZMPM_OK;
-    const unsigned nb = (unsigned)((P + XF_THREADS - 1) / XF_THREADS);
-    if (ctx->mixed)
-        k_explicit_stress<float, float><<<nb, XF_THREADS, 0, ctx->stream>>>(ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, P,
-            ctx->stress.as<float>(), ctx->scratch.as<float>());
-    else
-        k_explicit_stress<double, double><<<nb, XF_THREADS, 0, ctx->stream>>>(ctx->pd.as<double>(), ctx->pi.as<int32_t>(), ctx->Pcap, P,
-            ctx->stress.as<double>(), ctx->scratch.as<double>());
-    ++g_kernel_launches;
-    return ZMPM_OK;
-}
-
-// MLS = true: the MLS-MPM weight of particlesToGridWithForceHelper
-// (MpmSimulationBase.cpp:527-541), facc -= (S_p (x_i - x_p)) w_ip D^-1 with
-// D^-1 = 4 / dx^2, in place of S_p grad w_ip.
-template <class L, class TS, class TH, bool MLS = false>
+// The scatter of a stress buffer (ADMM's right-hand side), one CTA per group:
+// thread -> one cell of the page and every (blockDim/NPB)-th particle of it; the
+// cell's particles share one 27-node stencil, so their terms are summed in
+// registers and added to the shared window once per thread (FP32 keeps all 81
+// sums in registers, FP64 one force component per pass).  With nothing to gather
+// or compute per particle this beats records in shared memory (498k particles
+// FP32: 51 against 60 us; 31k FP64: 29 us, and 0.3 ms more per 20 with records).
+template <class L, class TS>
 __global__ void __launch_bounds__(XF_THREADS) k_force(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_nbr,
-    int64_t cap, const short4* __restrict__ base, double dx, const TH* __restrict__ frac, const TS* __restrict__ stress,
-    double* __restrict__ facc, const SolverScalars* __restrict__ sc, int gate = 0, const double* __restrict__ xpos = nullptr)
+    int64_t cap, const short4* __restrict__ base, double dx, const TS* __restrict__ frac, const TS* __restrict__ stress,
+    double* __restrict__ facc)
 {
-    if (gated_off(sc, gate)) return;
     constexpr int NPB = L::NPB;
     __shared__ __align__(16) TS acc[8 * 3 * NPB];
     __shared__ int32_t nbr[8];
@@ -346,10 +217,6 @@ __global__ void __launch_bounds__(XF_THREADS) k_force(const int32_t* __restrict_
     const TS inv_dx = TS(1.0 / dx);
     const int s0 = group_start[g], s1 = group_start[g + 1];
     build_cell_layout<L>(cl, base, s0, s1);
-    // Thread -> one cell of the page and every (blockDim/NPB)-th particle of
-    // it; the cell's particles share one 27-node stencil, so their terms are
-    // summed in registers and added to the shared window once per thread (FP32
-    // keeps all 81 sums in registers, FP64 one force component per pass).
     const int ce = threadIdx.x % NPB;
     const int lx = ce >> (L::YB + L::ZB), ly = (ce >> L::ZB) & (L::BY - 1), lz = ce & (L::BZ - 1);
     const int cnt = cl.cnt[ce], first = s0 + cl.start[ce];
@@ -363,38 +230,19 @@ __global__ void __launch_bounds__(XF_THREADS) k_force(const int32_t* __restrict_
             for (int c = 0; c < NCP; ++c) a[n][c] = TS(0);
         for (int r = threadIdx.x / NPB; r < cnt; r += blockDim.x / NPB) {
             const int s = first + r;
-            TS w[3][3], dwr[3][3], fr[3];
-            if (xpos) {
-                const short4 b = base[s];
+            TS w[3][3], dwr[3][3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) fr[d] = (TS)((1.0 / dx) * xpos[d * cap + s] - (double)((&b.x)[d]));
-            }
-            else
-#pragma unroll
-                for (int d = 0; d < 3; ++d) fr[d] = (TS)frac[d * cap + s];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) bspline(fr[d], w[d], dwr[d]);
+            for (int d = 0; d < 3; ++d) bspline(frac[d * cap + s], w[d], dwr[d]);
             TS row[NCP][3];
 #pragma unroll
             for (int c = 0; c < NCP; ++c)
 #pragma unroll
                 for (int q2 = 0; q2 < 3; ++q2) row[c][q2] = stress[(3 * (c0 + c) + q2) * cap + s];
-            if constexpr (MLS) {
-                const TS tdx = (TS)dx, dinv = TS(4.0 / (dx * dx));
-                for_stencil<L>(lx, ly, lz, w, dwr, inv_dx, [&](int, int, int i, int j, int k, TS wijk, const TS*) {
-                    const int n = 9 * i + 3 * j + k;
-                    const TS xm[3] = { ((TS)i - fr[0]) * tdx, ((TS)j - fr[1]) * tdx, ((TS)k - fr[2]) * tdx };
-                    const TS q = wijk * dinv;
+            for_stencil<L>(lx, ly, lz, w, dwr, inv_dx, [&](int, int, int i, int j, int k, TS, const TS* dw) {
+                const int n = 9 * i + 3 * j + k;
 #pragma unroll
-                    for (int c = 0; c < NCP; ++c) a[n][c] -= (row[c][0] * xm[0] + row[c][1] * xm[1] + row[c][2] * xm[2]) * q;
-                });
-            }
-            else
-                for_stencil<L>(lx, ly, lz, w, dwr, inv_dx, [&](int, int, int i, int j, int k, TS, const TS* dw) {
-                    const int n = 9 * i + 3 * j + k;
-#pragma unroll
-                    for (int c = 0; c < NCP; ++c) a[n][c] -= row[c][0] * dw[0] + row[c][1] * dw[1] + row[c][2] * dw[2];
-                });
+                for (int c = 0; c < NCP; ++c) a[n][c] -= row[c][0] * dw[0] + row[c][1] * dw[1] + row[c][2] * dw[2];
+            });
         }
         if (threadIdx.x / NPB < cnt) {
 #pragma unroll
@@ -412,6 +260,75 @@ __global__ void __launch_bounds__(XF_THREADS) k_force(const int32_t* __restrict_
     }
     __syncthreads();
     flush_window<3, 3, NPB>(acc, nbr, facc, nullptr);
+}
+
+// Explicit substep: FBasedMpmForceHelper::updateState (FBasedMpmForceHelper.cpp:
+// 44-64), S = V0 tau(F) = V0 P(F) F^T, plus V0 tau(Fe) for viscoelastic particles
+// (FElasticNonequilibratedBasedMpmForceHelper.h:39-60), in the pass that scatters
+// it (a stress kernel before it wrote 154 B per particle, the unused Hessian
+// scratch among them).  FP32 with the FP64 re-evaluation of near-degenerate SVDs.
+template <class T, bool MLS>
+struct ExplicitPhase1 {
+    const double* pd;
+    const int32_t* pi;
+    int64_t cap;
+    const T* frac;
+    T inv_dx;
+
+    template <int FS>
+    __device__ __forceinline__ void run(const void*, int64_t s, T* rc) const
+    {
+        T fr[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) fr[d] = frac[d * cap + s];
+        const int kind = pi[PI_KIND * cap + s];
+        M3<T> S = m3_zero<T>();
+        if (kind != ZMPM_MODEL_NONE) {
+            T scr[NS]; // the Hessian scratch, not kept
+            M3<T> F;
+#pragma unroll
+            for (int q = 0; q < 9; ++q) F.a[q] = (T)pd[(PD_F + q) * cap + s];
+            const ModelParams mp{ pd[PD_MU * cap + s], pd[PD_LAM * cap + s], pd[PD_KAPPA * cap + s], pd[PD_G * cap + s] };
+            const double V0 = pd[PD_VOL * cap + s];
+            bool degenerate = false;
+            S = model_update<T, T>(kind, mp, (T)V0, F, F, scr, 1, 0, sizeof(T) == 4 ? &degenerate : nullptr);
+            if constexpr (sizeof(T) == 4) {
+                if (degenerate) {
+                    M3<double> Fd;
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) Fd.a[q] = pd[(PD_F + q) * cap + s];
+                    S = m3_cast<T>(model_update<double, T>(kind, mp, V0, Fd, Fd, scr, 1, 0, nullptr));
+                }
+            }
+            if (pi[PI_VISCO * cap + s]) {
+                M3<double> Fe;
+#pragma unroll
+                for (int q = 0; q < 9; ++q) Fe.a[q] = pd[(PD_FE + q) * cap + s];
+                const ModelParams mv{ pd[PD_VMU * cap + s], pd[PD_VLAM * cap + s], 0.0, 1.0 };
+                const M3<double> Se = model_update<double, T>(ZMPM_MODEL_STVK_HENCKY_ISOTROPIC, mv, V0, Fe, Fe, scr, 1, 0, nullptr);
+#pragma unroll
+                for (int q = 0; q < 9; ++q) S.a[q] += (T)Se.a[q];
+            }
+        }
+        force_record<T, MLS, FS>(S, fr, inv_dx, rc);
+    }
+};
+
+template <class L, class T, bool MLS>
+using ForceSmem = GroupSmem<L, T, void, MLS ? 15 : 12, 3>;
+constexpr int FORCE_PIECE = 96; // fixed cost of a piece in particles
+
+template <class L, class T, bool MLS, class Phase1>
+__global__ void __launch_bounds__(FUSED_THREADS, ForceSmem<L, T, MLS>::CTAS) k_force_fused(GroupArgs ga, Phase1 p1, double* __restrict__ facc,
+    int32_t* __restrict__ flags)
+{
+    using Scatter = typename std::conditional<MLS, AffineScatter<T, false>, RowsScatter<T>>::type;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    ForceSmem<L, T, MLS>& sm = *reinterpret_cast<ForceSmem<L, T, MLS>*>(smem_raw);
+    group_smem_init(sm);
+    Share share(ga);
+    int ph = 0;
+    group_share<L, T, void, Scatter, 3>(sm, ga, share, nullptr, facc, nullptr, flags, ph, p1);
 }
 
 // ------------------------------------------------------- fused products ----
@@ -728,22 +645,19 @@ __global__ void __launch_bounds__(XF_THREADS, sizeof(T) == 4 ? 4 : 3) k_g2p(cons
 }
 
 // ------------------------------------------------------------- launchers --
-template <class L>
+template <class L, class T>
 static int p2g_impl(Ctx* ctx)
 {
-    const int64_t G = ctx->G;
-    if (G == 0) return ZMPM_OK;
-    if (ctx->mixed)
-        return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, P2G_PIECE), sizeof(P2gSmem<L, float>), k_p2g_fused<L, float>, group_args(ctx, P2G_PIECE),
-            ctx->pd.as<double>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->gm.as<double>(), ctx->gmv.as<double>(),
-            ctx->frac.as<float>(), &ctx->counters.as<DevCounters>()->flags);
-    else
-        k_p2g_reg<L, double, 2><<<(unsigned)G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(),
-            ctx->pd.as<double>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->gm.as<double>(), ctx->gmv.as<double>(), ctx->frac.as<double>());
-    ++g_kernel_launches;
-    return ZMPM_OK;
+    if (ctx->G == 0) return ZMPM_OK;
+    return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, P2G_PIECE), sizeof(P2gSmem<L, T>), k_p2g_fused<L, T>,
+        group_args(ctx, P2G_PIECE), ctx->pd.as<double>(), ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->gm.as<double>(),
+        ctx->gmv.as<double>(), ctx->frac.as<T>(), &ctx->counters.as<DevCounters>()->flags);
 }
-int launch_p2g(Ctx* ctx) { return ctx->layout == 1 ? p2g_impl<Layout244>(ctx) : p2g_impl<Layout444>(ctx); }
+int launch_p2g(Ctx* ctx)
+{
+    if (ctx->mixed) return ctx->layout == 1 ? p2g_impl<Layout244, float>(ctx) : p2g_impl<Layout444, float>(ctx);
+    return ctx->layout == 1 ? p2g_impl<Layout244, double>(ctx) : p2g_impl<Layout444, double>(ctx);
+}
 
 template <class L>
 static int update_impl(Ctx* ctx, bool gated)
@@ -807,26 +721,43 @@ int launch_hvp(Ctx* ctx, const double* x, double* out, bool fp32)
     return ctx->layout == 1 ? hvp_impl<Layout244>(ctx, x, out) : hvp_impl<Layout444>(ctx, x, out);
 }
 
-template <class L, class TH>
-static int force_scatter_impl(Ctx* ctx, double* out, bool mls)
+template <class L, class T, bool MLS, class Phase1>
+static int force_impl(Ctx* ctx, const Phase1& p1, double* out)
 {
-    if (mls)
-        k_force<L, TH, TH, true><<<(unsigned)ctx->G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(),
-            ctx->Pcap, ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<TH>(), ctx->stress.as<TH>(), out, nullptr);
-    else
-        k_force<L, TH, TH><<<(unsigned)ctx->G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(), ctx->Pcap,
-            ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<TH>(), ctx->stress.as<TH>(), out, nullptr);
+    return launch_resident(ctx, ctx->stream, false, useful_ctas(ctx, FORCE_PIECE), sizeof(ForceSmem<L, T, MLS>),
+        k_force_fused<L, T, MLS, Phase1>, group_args(ctx, FORCE_PIECE), p1, out, &ctx->counters.as<DevCounters>()->flags);
+}
+// out -= sum_p stress_p grad w_ip with `stress` in the HVP precision.
+template <class L, class T>
+static int force_scatter_impl(Ctx* ctx, double* out)
+{
+    k_force<L, T><<<(unsigned)ctx->G, XF_THREADS, 0, ctx->stream>>>(ctx->group_start.as<int32_t>(), ctx->group_nbr.as<int32_t>(), ctx->Pcap,
+        ctx->base.as<short4>(), ctx->cfg.dx, ctx->frac.as<T>(), ctx->stress.as<T>(), out);
     ++g_kernel_launches;
     return ZMPM_OK;
 }
-// out -= sum_p stress_p grad w_ip with `stress` in the HVP precision (the MLS
-// weight when mls).
-int launch_force_scatter(Ctx* ctx, double* out, bool mls)
+int launch_force_scatter(Ctx* ctx, double* out)
+{
+    if (!ctx->G) return ZMPM_OK;
+    if (ctx->mixed) return ctx->layout == 1 ? force_scatter_impl<Layout244, float>(ctx, out) : force_scatter_impl<Layout444, float>(ctx, out);
+    return ctx->layout == 1 ? force_scatter_impl<Layout244, double>(ctx, out) : force_scatter_impl<Layout444, double>(ctx, out);
+}
+// out -= the explicit substep's forces (after P2G, which forms the fractions).
+template <class L, class T>
+static int explicit_force_impl(Ctx* ctx, double* out, bool mls)
+{
+    const double* pd = ctx->pd.as<double>();
+    const int32_t* pi = ctx->pi.as<int32_t>();
+    const T inv_dx = T(1.0 / ctx->cfg.dx);
+    if (mls) return force_impl<L, T, true>(ctx, ExplicitPhase1<T, true>{ pd, pi, ctx->Pcap, ctx->frac.as<T>(), inv_dx }, out);
+    return force_impl<L, T, false>(ctx, ExplicitPhase1<T, false>{ pd, pi, ctx->Pcap, ctx->frac.as<T>(), inv_dx }, out);
+}
+int launch_explicit_force(Ctx* ctx, double* out, bool mls)
 {
     if (!ctx->G) return ZMPM_OK;
     if (ctx->mixed)
-        return ctx->layout == 1 ? force_scatter_impl<Layout244, float>(ctx, out, mls) : force_scatter_impl<Layout444, float>(ctx, out, mls);
-    return ctx->layout == 1 ? force_scatter_impl<Layout244, double>(ctx, out, mls) : force_scatter_impl<Layout444, double>(ctx, out, mls);
+        return ctx->layout == 1 ? explicit_force_impl<Layout244, float>(ctx, out, mls) : explicit_force_impl<Layout444, float>(ctx, out, mls);
+    return ctx->layout == 1 ? explicit_force_impl<Layout244, double>(ctx, out, mls) : explicit_force_impl<Layout444, double>(ctx, out, mls);
 }
 
 // out += sum_p (grad(x)_p B_p) grad w_ip (ADMM's global operator).
