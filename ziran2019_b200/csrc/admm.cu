@@ -4,20 +4,17 @@
 // The reference assembles the global matrix M + sum_p rho omega^2 dt^2
 // (Fn^T grad w_ip)(Fn^T grad w_jp)^T as a 125-entry stencil per node
 // (initMultiplierAndPreconditioner, :407-505) and multiplies it in MINRES.
-// Here the product is matrix-free: with B_p = rho dt^2 (omega_0^2 Fn Fn^T +
-// omega_1^2 Fe Fe^T) (6 numbers per particle),
-//     (A x)_i = m_i x_i + sum_p (grad x_p B_p) grad w_ip,  grad x_p = sum_j x_j grad w_jp^T,
-// the same gather -> 3x3 -> scatter shape as the Newton Hessian product, so it
-// runs through the same per-group product (hvp.cuh, AdmmOpModel): k_op_fused
-// for the right-hand side's product, the persistent MINRES for the solve.
-// Per product that is 6 numbers per particle instead of 125 values + 125
-// indices per node.
+// With B_p = rho dt^2 (omega_0^2 Fn Fn^T + omega_1^2 Fe Fe^T) (6 numbers per
+// particle) that operator is
+//     (A x)_i = m_i x_i + sum_p (grad x_p B_p) grad w_ip,  grad x_p = sum_j x_j grad w_jp^T.
+// stencil.cu sums it into node rows once per substep; where the particles are too
+// sparse for rows it runs matrix-free through the product of hvp.cuh (AdmmOpModel).
 //
 // Kernels
 //  k_admm_dvinit   dv_i = sum_p last_dv_p w_ip, w_i = sum_p w_ip (initStep :304-320)
 //  k_admm_init     F = (I + dt grad(vn+dv)) Fn (and Fe), grad vn, omega
 //                  (initOmega :222-274), y <- y omega_old / omega, B
-//  k_admm_pre      preconditioner m_i + sum_p grad w^T B grad w (:477-503)
+//  k_admm_pre      preconditioner m_i + sum_p grad w^T B grad w (:477-503), matrix-free
 //  k_admm_local    FStepSolve (:507-615) for F and Fe, then the dvStep
 //                  right-hand side stress dt rho omega^2 bFu Fn^T (:163-205)
 //  k_admm_dual     uStep (:638-671)
