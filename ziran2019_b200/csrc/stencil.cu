@@ -9,7 +9,7 @@
 // (dz + 2) of a page's nodes is contiguous.
 //
 // Why assembled: the matrix-free product (hvp.cuh, AdmmOpModel) runs every
-// particle's gather and scatter per product, about 0.23 ns per particle (0.11
+// particle's gather and scatter per product, about 0.19 ns per particle (0.096
 // ms at 498k particles); the stencil reads 125 coefficients per node slot
 // from L2 and needs no atomics, no accumulator pass and one grid barrier less
 // per iteration.  The product is bound by the coefficient reads.
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_stencil(NodeGeom ng, in
 
 // -------------------------------------------------------------- host side --
 // The stencil costs its coefficient reads per page (0.2 ns per KB measured
-// from L2 and HBM), the matrix-free product 0.23 ns per particle and about 192
+// from L2 and HBM), the matrix-free product 0.19 ns per particle and about 192
 // particles' worth per group: the stencil is taken where its bytes are below
 // 1 KB per such unit (dense scenes need about 150 B; a spray of single
 // particles, 500 KB each, stays matrix-free).
