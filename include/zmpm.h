@@ -493,6 +493,11 @@ int zmpm_residual(zmpm_ctx* ctx, const double* dv, double* residual, double* nor
    fp32 != 0 evaluates the Hessian-vector product in FP32 (MIXED contexts). */
 int zmpm_multiply(zmpm_ctx* ctx, const double* x, double* b, int32_t fp32);
 
+/* Makes the nth device allocation of the calling thread from here on fail once,
+   as an exhausted device would (0: none does).  The call it fails in returns
+   ZMPM_CUDA_ERROR and the context stays usable. */
+int zmpm_fail_allocation(int32_t nth);
+
 /* --------------------------------------------------- allocation-free ----- */
 /* Largest particle count zmpm_sort_keys_noalloc accepts. */
 #define ZMPM_NOALLOC_MAX_PARTICLES 262144

@@ -191,6 +191,7 @@ _PRODUCT_ONLY = {
     "grid_to_particles": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(Stats)]),
     "apply_plasticity": (C.c_int, [C.c_void_p]),
     "set_spin_limit": (C.c_int, [C.c_void_p, C.c_int64]),
+    "fail_allocation": (C.c_int, [C.c_int32]),
 }
 
 

@@ -989,6 +989,13 @@ int zmpm_set_spin_limit(zmpm_ctx* ctx, int64_t polls)
     return ZMPM_OK;
 }
 
+int zmpm_fail_allocation(int32_t nth)
+{
+    if (nth < 0) return ZMPM_BAD_ARG;
+    g_fail_allocation = nth;
+    return ZMPM_OK;
+}
+
 int zmpm_set_profiling(zmpm_ctx* ctx, int32_t on)
 {
     if (!ctx) return ZMPM_BAD_ARG;

@@ -432,7 +432,8 @@ __global__ void __launch_bounds__(1024) k_number(const int4* __restrict__ group_
     }
 }
 
-// The radix way (see the top of the file); dc is zeroed and the page tables are clean.
+// The radix way (see the top of the file); dc is zeroed and the page tables are
+// clean, but counted as dirty until the pass is complete.
 template <class L, class KT>
 static int binning_radix(Ctx* ctx)
 {
@@ -505,6 +506,7 @@ static int binning_radix(Ctx* ctx)
     k_group_nbr<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->page_block.as<int32_t>(), first, ctx->group_nbr.as<int32_t>(), nullptr);
     ++g_kernel_launches;
     ZMPM_CUDA(cudaGetLastError());
+    ctx->tables_dirty = false;
     ctx->binned = true;
     return ZMPM_OK;
 }
@@ -516,6 +518,7 @@ static int binning_impl(Ctx* ctx)
     const int64_t P = ctx->P, cap = ctx->Pcap;
     PageDims pdims{ ctx->pages[0], ctx->pages[1], ctx->pages[2] };
     DevCounters* dc = ctx->counters.as<DevCounters>();
+    ctx->binned = false;
     ZMPM_CUDA(cudaMemsetAsync(dc, 0, sizeof(DevCounters), st));
     if (P == 0) {
         ctx->G = ctx->B = 0;
@@ -534,6 +537,14 @@ static int binning_impl(Ctx* ctx)
     int32_t* cnt = ctx->page_count.as<int32_t>();
     int32_t* first = ctx->page_first.as<int32_t>();
     short4* base_old = ctx->base_by_id.as<short4>(); // here by old slot
+    // A pass marks both page tables and clears the marks at its end; one that
+    // stopped in between (a failed allocation) left them, and a pass over such
+    // tables would miss pages and place particles out of range.
+    if (ctx->tables_dirty) {
+        ZMPM_CUDA(cudaMemsetAsync(cnt, 0, ctx->table_size * sizeof(int32_t), st));
+        ZMPM_CUDA(cudaMemsetAsync(first, 0x7f, ctx->table_size * sizeof(int32_t), st));
+    }
+    ctx->tables_dirty = true;
     k_count<L, KT><<<nblk(P), BIN_THREADS, 0, st>>>(ctx->pdf(PD_X), cap, P, 1.0 / ctx->cfg.dx, 1.0f / (float)ctx->cfg.dx, base_old, cnt, list,
         pdims, dc);
     k_pages<<<std::min(nblk(8 * P), 1024u), BIN_THREADS, 0, st>>>(list, pdims, cnt, list_cnt, first, dc);
@@ -547,6 +558,7 @@ static int binning_impl(Ctx* ctx)
         ++g_kernel_launches;
         ZMPM_CUDA(cudaGetLastError());
         if (out) {
+            ctx->tables_dirty = false;
             ctx->err = "a particle's stencil leaves the grid (raise grid_log2 or move the scene)";
             return ZMPM_OUT_OF_GRID;
         }
@@ -576,6 +588,7 @@ static int binning_impl(Ctx* ctx)
     k_group_nbr<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->page_block.as<int32_t>(), first, ctx->group_nbr.as<int32_t>(), cnt);
     g_kernel_launches += 7;
     ZMPM_CUDA(cudaGetLastError());
+    ctx->tables_dirty = false;
     ctx->binned = true;
     return ZMPM_OK;
 }

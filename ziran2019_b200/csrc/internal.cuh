@@ -17,6 +17,8 @@ namespace zmpm {
 // Kernels launched by this library on the calling host thread (reported per
 // substep in zmpm_stats.kernel_launches).
 extern thread_local int64_t g_kernel_launches;
+// Device allocations of this thread until one fails (0: none does), zmpm_fail_allocation.
+extern thread_local int32_t g_fail_allocation;
 
 // ------------------------------------------------------------ primitives --
 int64_t scan_scratch_elems(int64_t n);
@@ -37,9 +39,15 @@ struct DBuf {
         if (p) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        if (g_fail_allocation > 0 && --g_fail_allocation == 0) return cudaErrorMemoryAllocation;
         size_t want = n + n / 4 + 256;
         cudaError_t e = cudaMalloc(&p, want);
-        if (e == cudaSuccess) bytes = want;
+        if (e == cudaSuccess)
+            bytes = want;
+        else {
+            p = nullptr;
+            cudaGetLastError(); // returned here: not an error of the next call
+        }
         return e;
     }
     void release()
@@ -187,6 +195,7 @@ struct Ctx {
     DBuf group_start, group_page, group_nbr, emit_flag, emit_scan;
     DBuf group_cells;                     // GroupCells record per group (xfer.cuh)
     DBuf page_first, page_block, page_count; // dense page tables
+    bool tables_dirty = false;            // a binning pass that failed may have left marks in page_first and page_count
     DBuf page_list;                       // occupied pages in any order, then their particle counts (binning)
     DBuf block_page, block_index;         // per page: packed coords, page index
     int64_t G = 0, B = 0, N = 0;

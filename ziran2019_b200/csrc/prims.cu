@@ -12,6 +12,7 @@
 namespace zmpm {
 
 thread_local int64_t g_kernel_launches = 0;
+thread_local int32_t g_fail_allocation = 0;
 
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
