@@ -417,7 +417,10 @@ int zmpm_adjoint_substep(zmpm_ctx* ctx, double dt, const zmpm_solver* s, double 
 
 /* Device-resident checkpoints of the full particle state and time (for
    checkpointed adjoint rollouts).  slot >= 0; a slot is allocated on first
-   save and kept until zmpm_destroy. */
+   save and kept until zmpm_destroy.  A load puts back every particle field,
+   the Lame parameters of the time of the save included; it is refused
+   (ZMPM_BAD_ARG) between an edit of the scene, zmpm_set_lame too, and the next
+   call that runs on the device. */
 int zmpm_checkpoint_save(zmpm_ctx* ctx, int32_t slot);
 int zmpm_checkpoint_load(zmpm_ctx* ctx, int32_t slot);
 

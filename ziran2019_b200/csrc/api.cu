@@ -121,6 +121,7 @@ namespace zmpm {
 // Puts the host scene on the device (first use) with slot = particle index.
 int upload(Ctx* ctx)
 {
+    ctx->edited = false;
     if (ctx->uploaded) return ZMPM_OK;
     const int64_t P = ctx->P;
     const int64_t cap = std::max<int64_t>(P, 1);
@@ -706,6 +707,7 @@ int zmpm_set_lame(zmpm_ctx* ctx, int64_t lo, int64_t hi, const double* mu, const
             ZMPM_CUDA(cudaGetLastError());
             ZMPM_CUDA(cudaStreamSynchronize(ctx->stream));
         }
+        ctx->edited = true;
         ctx->binned = false;
         ctx->implicit_ready = false;
         ctx->phase = 0; // an edit ends a substep split into phases
@@ -1472,8 +1474,8 @@ int zmpm_checkpoint_save(zmpm_ctx* ctx, int32_t slot)
 int zmpm_checkpoint_load(zmpm_ctx* ctx, int32_t slot)
 {
     if (!ctx || slot < 0 || (size_t)slot >= ctx->ckpt_pd.size() || ctx->ckpt_P[slot] < 0) return ZMPM_BAD_ARG;
-    if (ctx->ckpt_P[slot] != ctx->P * 1000 + ctx->pd_active || !ctx->uploaded) {
-        ctx->err = "the checkpoint was saved with a different particle set";
+    if (ctx->ckpt_P[slot] != ctx->P * 1000 + ctx->pd_active || !ctx->uploaded || ctx->edited) {
+        ctx->err = "the checkpoint was saved with a different particle set, or the scene was edited and has not run since";
         return ZMPM_BAD_ARG;
     }
     cudaSetDevice(ctx->device);

@@ -149,6 +149,7 @@ struct Ctx {
     // host copy of the scene until the first upload
     int64_t P = 0;
     bool uploaded = false;
+    bool edited = false;        // edited on the device since the last call that ran on it: checkpoints do not load, as after any edit
     std::vector<double> hx, hv, hC, hF, hcrack, hm, hvol, hmu, hlam, hkappa, hg, hys, hxi, hfs, hpfc, hpfk, hsigf, hlogjp;
     std::vector<uint8_t> hkind, hpkind, hdamage, hvisco;
     std::vector<int32_t> hbroken;

@@ -552,6 +552,8 @@ class MpmSimulation:
         self._call("checkpoint_save", int(slot))
 
     def checkpointLoad(self, slot):
+        """Puts back every particle field as saved, the moduli included; refused right after an edit (setYoungsModulus
+        too), until a call has run on the device."""
         self._call("checkpoint_load", int(slot))
 
     def setYoungsModulus(self, E, nu, lower=0, upper=None):
