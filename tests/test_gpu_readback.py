@@ -1,5 +1,5 @@
-"""Particle fields between host arrays and the device: sizes around the pinned
-blocks of large transfers, every slot order, and Lame parameters set in place."""
+"""Particle fields between host arrays and the device: sizes from one particle
+to many, every slot order, and Lame parameters set in place."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 DX = 1.0 / 64
 
 
-# bytes of x (24 n) and C (72 n) around 2 MB (where the pinned blocks take over), 4 MB (one block) and several blocks
+# bytes of x (24 n) and C (72 n) around 2, 4 and 6 MB (whole pages and a few bytes off), and large
 @pytest.mark.parametrize("n", [1, 29127, 29128, 58254, 58255, 87381, 87382, 174763, 400003])
 def test_round_trip(cuda_lib, n):
     rng = np.random.default_rng(n)

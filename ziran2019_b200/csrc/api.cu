@@ -1,14 +1,16 @@
 // C ABI of the library (include/zmpm.h): context lifecycle, scene plugins,
 // state I/O, the substep and the test hooks.  No exception crosses the
 // boundary; every entry point returns a zmpm_status_code.
+#include <sys/mman.h>
+
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <cstdlib>
+#include <exception>
 #include <limits>
-#include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 
 #include "internal.cuh"
@@ -32,70 +34,106 @@ cudaError_t d2h_sync(Ctx* ctx, void* dst, const void* src, size_t bytes)
     return cudaStreamSynchronize(ctx->stream);
 }
 
-// Device -> caller's memory of a finished array, complete on return.  A plain
-// copy to pageable memory runs at 6 GB/s here (one thread of the driver copies,
-// and takes the page faults of a fresh destination); arrays of a few MB and
-// more go through two pinned blocks instead, one filling over PCIe while
-// threads empty the other.  192 MB (x, v, C, F of 1M particles) into fresh
-// memory: 13-33 -> 12 ms, by host.  The blocks belong to the process, because
-// pinning 8 MB takes about 10 ms: made for the first transfer that wants them,
-// freed with the last context, used by one thread at a time (another thread's
-// transfer meanwhile takes the plain copy).
-constexpr size_t PIN_BLOCK = 4 << 20, PIN_FROM = 2 << 20;
-constexpr int PIN_THREADS = 8;
-struct PinBlocks {
-    std::mutex m;
-    void* p = nullptr;
-    int contexts = 0;
-};
-PinBlocks g_pin;
+// Arrays on their way to the caller's memory.  The copies themselves run at the
+// link's rate (21 GB/s into pageable memory, 53 GB/s into page-locked), but a
+// freshly allocated destination takes its page faults inside them, on the one
+// thread of the driver that copies: 192 MB then took 38 ms in 2 MB pages and 88
+// ms in 4 KB pages instead of 9.  So threads touch the pages of such arrays first,
+// running ahead of the copies array by array: 15 and 55 ms (16 host cores).
+// Memory that has its pages, page-locked memory and small arrays (4 MB: 0.8 ms
+// plain, 1.0 touched) are copied as they are.
+constexpr size_t TOUCH_FROM = 8 << 20, TOUCH_CHUNK = 2 << 20, PAGE_BYTES = 4096;
+constexpr int TOUCH_THREADS = 8, READ_MAX = 4;
 
-void copy_threaded(char* dst, const char* src, size_t bytes)
+// Ordinary memory of this process with a page missing at its start, middle or end.
+bool lacks_pages(char* dst, size_t bytes)
 {
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int n = (int)std::min<size_t>(std::min<size_t>(PIN_THREADS, hw ? hw : 1), bytes / (256 << 10) + 1);
-    std::thread t[PIN_THREADS];
-    const size_t per = ((bytes / n) + 4095) & ~(size_t)4095;
-    int started = 0;
-    for (int i = 1; i < n; ++i) {
-        const size_t a = std::min(bytes, per * i), b = i + 1 == n ? bytes : std::min(bytes, per * (i + 1));
-        if (a >= b) continue;
+    if (bytes < TOUCH_FROM) return false;
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, dst) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (attr.type != cudaMemoryTypeUnregistered) return false;
+    const uintptr_t lo = ((uintptr_t)dst + PAGE_BYTES - 1) / PAGE_BYTES, hi = ((uintptr_t)dst + bytes) / PAGE_BYTES - 1;
+    for (const uintptr_t page : { lo, (lo + hi) / 2, hi }) {
+        unsigned char in = 1;
+        if (mincore((void*)(page * PAGE_BYTES), PAGE_BYTES, &in) != 0) return false;
+        if (!(in & 1)) return true;
+    }
+    return false;
+}
+
+// Touches the pages of the arrays added, in their order, from TOUCH_THREADS - 1
+// threads and the caller's; the threads end with the object.
+class PageToucher {
+public:
+    ~PageToucher()
+    {
+        next = chunks; // nothing more to take
+        for (int i = 0; i < started; ++i) thread[i].join();
+    }
+    void add(int a, char* dst, size_t bytes)
+    {
+        lo[a] = dst;
+        hi[a] = dst + bytes;
+        const size_t n = ((uintptr_t)hi[a] + TOUCH_CHUNK - 1) / TOUCH_CHUNK - (uintptr_t)dst / TOUCH_CHUNK;
+        left[a] = (int64_t)n;
+        chunks += n;
+    }
+    void start()
+    {
+        if (chunks == 0) return;
+        const unsigned hw = std::thread::hardware_concurrency();
+        const int n = std::min<int>(TOUCH_THREADS - 1, hw ? (int)hw - 1 : 0);
         try {
-            t[started] = std::thread([=] { std::memcpy(dst + a, src + a, b - a); });
-            ++started;
+            for (; started < n; ++started)
+                thread[started] = std::thread([this] {
+                    while (one()) {}
+                });
         }
-        catch (const std::system_error&) { // no thread to be had: this one copies
-            std::memcpy(dst + a, src + a, b - a);
+        catch (const std::exception&) { // no thread to be had: the others do it
         }
     }
-    std::memcpy(dst, src, n == 1 ? bytes : std::min(bytes, per));
-    for (int i = 0; i < started; ++i) t[i].join();
-}
+    // Returns once the pages of array a are there.
+    void wait(int a)
+    {
+        while (left[a] > 0)
+            if (!one()) std::this_thread::yield();
+    }
 
-cudaError_t copy_out(Ctx* ctx, void* dst, const void* src, size_t bytes)
-{
-    std::unique_lock<std::mutex> lock(g_pin.m, std::defer_lock);
-    if (bytes < PIN_FROM || !lock.try_lock()) return d2h_sync(ctx, dst, src, bytes);
-    if (!g_pin.p && cudaHostAlloc(&g_pin.p, 2 * PIN_BLOCK, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError(); // no pinned memory: the plain copy
-        g_pin.p = nullptr;
-        return d2h_sync(ctx, dst, src, bytes);
+private:
+    bool one() // touches the next chunk; false when none is left
+    {
+        size_t k = next.fetch_add(1);
+        if (k >= chunks) return false;
+        for (int a = 0; a < READ_MAX; ++a) {
+            if (!lo[a]) continue;
+            const uintptr_t first = (uintptr_t)lo[a] / TOUCH_CHUNK;
+            const size_t n = ((uintptr_t)hi[a] + TOUCH_CHUNK - 1) / TOUCH_CHUNK - first;
+            if (k >= n) {
+                k -= n;
+                continue;
+            }
+            char* p = std::max(lo[a], (char*)((first + k) * TOUCH_CHUNK));
+            char* const e = std::min(hi[a], (char*)((first + k + 1) * TOUCH_CHUNK));
+            while (p < e) {
+                volatile char* v = p;
+                *v = *v; // the bytes stay as they are
+                p = (char*)(((uintptr_t)p / PAGE_BYTES + 1) * PAGE_BYTES);
+            }
+            --left[a];
+            return true;
+        }
+        return false;
     }
-    char* block[2] = { static_cast<char*>(g_pin.p), static_cast<char*>(g_pin.p) + PIN_BLOCK };
-    const size_t n = (bytes + PIN_BLOCK - 1) / PIN_BLOCK;
-    auto size = [&](size_t k) { return std::min(PIN_BLOCK, bytes - k * PIN_BLOCK); };
-    cudaError_t e = cudaMemcpyAsync(block[0], src, size(0), cudaMemcpyDeviceToHost, ctx->stream);
-    for (size_t k = 0; k < n && e == cudaSuccess; ++k) {
-        e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) break;
-        if (k + 1 < n)
-            e = cudaMemcpyAsync(block[(k + 1) & 1], static_cast<const char*>(src) + (k + 1) * PIN_BLOCK, size(k + 1), cudaMemcpyDeviceToHost,
-                ctx->stream);
-        copy_threaded(static_cast<char*>(dst) + k * PIN_BLOCK, block[k & 1], size(k));
-    }
-    if (e != cudaSuccess) cudaStreamSynchronize(ctx->stream); // nothing may still write the blocks
-    return e;
-}
+    char *lo[READ_MAX] = {}, *hi[READ_MAX] = {};
+    std::atomic<int64_t> left[READ_MAX] = {};
+    size_t chunks = 0;
+    std::atomic<size_t> next{ 0 };
+    std::thread thread[TOUCH_THREADS];
+    int started = 0;
+};
 
 int64_t bitlen(uint64_t v)
 {
@@ -382,40 +420,58 @@ int device_set(Ctx* ctx, const double* x, const double* v, const double* C, cons
     return ZMPM_OK;
 }
 
-// Fields [f, f + ncomp) of the double pool to a host array in particle-index
-// order.  The pool must be on the device and the fields active.
-int get_field(Ctx* ctx, int f, int ncomp, double* dst)
+// Device fields to host arrays in particle-index order, complete on return.
+// The pools must be on the device and the fields active; arrays not asked for
+// are null.
+struct FieldOut {
+    const void* field; // component 0, [ncomp][Pcap]
+    int ncomp;
+    size_t elem;       // 8: double, 4: int32_t
+    void* dst;
+};
+int read_fields(Ctx* ctx, const FieldOut* f, int n)
 {
     const int64_t P = ctx->P;
-    if (P == 0 || !dst) return ZMPM_OK;
-    ZMPM_CUDA(ctx->stage.ensure((size_t)ncomp * P * sizeof(double)));
-    k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, ctx->stream>>>(ctx->stage.as<double>(), ncomp, P, ctx->Pcap,
-        ctx->slot_of_id.as<int32_t>(), ctx->pdf(f));
-    ++g_kernel_launches;
+    if (P == 0) return ZMPM_OK;
+    size_t off[READ_MAX + 1] = {};
+    for (int a = 0; a < n; ++a) off[a + 1] = off[a] + (f[a].dst ? ((size_t)f[a].ncomp * P * f[a].elem + 15) / 16 * 16 : 0);
+    if (off[n] == 0) return ZMPM_OK;
+    ZMPM_CUDA(ctx->stage.ensure(off[n]));
+    char* st = ctx->stage.as<char>();
+    const unsigned grid = (unsigned)((P + 255) / 256);
+    const int32_t* slot = ctx->slot_of_id.as<int32_t>();
+    PageToucher pages;
+    for (int a = 0; a < n; ++a) {
+        if (!f[a].dst) continue;
+        const size_t bytes = (size_t)f[a].ncomp * P * f[a].elem;
+        if (f[a].elem == sizeof(double))
+            k_fields_to_host<<<grid, 256, 0, ctx->stream>>>((double*)(st + off[a]), f[a].ncomp, P, ctx->Pcap, slot, (const double*)f[a].field);
+        else
+            k_fields_to_host<<<grid, 256, 0, ctx->stream>>>((int32_t*)(st + off[a]), f[a].ncomp, P, ctx->Pcap, slot, (const int32_t*)f[a].field);
+        ++g_kernel_launches;
+        if (lacks_pages((char*)f[a].dst, bytes)) pages.add(a, (char*)f[a].dst, bytes);
+    }
     ZMPM_CUDA(cudaGetLastError());
-    ZMPM_CUDA(copy_out(ctx, dst, ctx->stage.p, (size_t)ncomp * P * sizeof(double)));
+    pages.start();
+    for (int a = 0; a < n; ++a) {
+        if (!f[a].dst) continue;
+        pages.wait(a);
+        ZMPM_CUDA(cudaMemcpyAsync(f[a].dst, st + off[a], (size_t)f[a].ncomp * P * f[a].elem, cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    ZMPM_CUDA(cudaStreamSynchronize(ctx->stream));
     return ZMPM_OK;
 }
-int get_field(Ctx* ctx, int f, int32_t* dst)
+int read_field(Ctx* ctx, int f, int ncomp, double* dst)
 {
-    const int64_t P = ctx->P;
-    if (P == 0 || !dst) return ZMPM_OK;
-    ZMPM_CUDA(ctx->stage.ensure(P * sizeof(int32_t)));
-    k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, ctx->stream>>>(ctx->stage.as<int32_t>(), 1, P, ctx->Pcap,
-        ctx->slot_of_id.as<int32_t>(), ctx->pif(f));
-    ++g_kernel_launches;
-    ZMPM_CUDA(cudaGetLastError());
-    ZMPM_CUDA(copy_out(ctx, dst, ctx->stage.p, P * sizeof(int32_t)));
-    return ZMPM_OK;
+    const FieldOut out = { ctx->pdf(f), ncomp, sizeof(double), dst };
+    return read_fields(ctx, &out, 1);
 }
 
 int device_get(Ctx* ctx, double* x, double* v, double* C, double* F)
 {
-    int rc = get_field(ctx, PD_X, 3, x);
-    if (!rc) rc = get_field(ctx, PD_V, 3, v);
-    if (!rc) rc = get_field(ctx, PD_C, 9, C);
-    if (!rc) rc = get_field(ctx, PD_F, 9, F);
-    return rc;
+    const FieldOut out[4] = { { ctx->pdf(PD_X), 3, sizeof(double), x }, { ctx->pdf(PD_V), 3, sizeof(double), v },
+        { ctx->pdf(PD_C), 9, sizeof(double), C }, { ctx->pdf(PD_F), 9, sizeof(double), F } };
+    return read_fields(ctx, out, 4);
 }
 
 int check_ready(Ctx* ctx)
@@ -563,10 +619,6 @@ int zmpm_create(const zmpm_config* cfg, zmpm_ctx** out)
     cudaMemset(ctx->scal.p, 0, sizeof(SolverScalars));
     // the context's stream does not order itself after the legacy stream's memsets
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail(e);
-    {
-        std::lock_guard<std::mutex> lock(g_pin.m);
-        ++g_pin.contexts; // given back in zmpm_destroy
-    }
     *out = ctx;
     return ZMPM_OK;
 }
@@ -588,13 +640,6 @@ int zmpm_destroy(zmpm_ctx* ctx)
     for (auto* v : { &ctx->ckpt_pd, &ctx->ckpt_pi, &ctx->ckpt_sid })
         for (auto& b : *v) b.release();
     ctx->stage.release();
-    {
-        std::lock_guard<std::mutex> lock(g_pin.m);
-        if (--g_pin.contexts == 0 && g_pin.p) {
-            cudaFreeHost(g_pin.p);
-            g_pin.p = nullptr;
-        }
-    }
     for (cudaEvent_t e : ctx->hvp_ev) cudaEventDestroy(e);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -797,7 +842,7 @@ int zmpm_get_log_jp(zmpm_ctx* ctx, double* log_jp)
 {
     if (!ctx || !log_jp) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    if (ctx->uploaded) return get_field(ctx, PD_LOGJP, 1, log_jp);
+    if (ctx->uploaded) return read_field(ctx, PD_LOGJP, 1, log_jp);
     std::memcpy(log_jp, ctx->hlogjp.data(), ctx->P * sizeof(double));
     return ZMPM_OK;
 }
@@ -822,7 +867,7 @@ int zmpm_get_damage(zmpm_ctx* ctx, double* c)
 {
     if (!ctx || !c) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    if (ctx->uploaded) return get_field(ctx, PD_PF_C, 1, c);
+    if (ctx->uploaded) return read_field(ctx, PD_PF_C, 1, c);
     for (int64_t i = 0; i < ctx->P; ++i) c[i] = ctx->hpfc[i];
     return ZMPM_OK;
 }
@@ -887,11 +932,9 @@ int zmpm_get_phase_field(zmpm_ctx* ctx, double* c, double* H, double* pf_Fp, dou
     if (!ctx) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
     if (ctx->uploaded && ctx->pd_active >= PD_PF_END) {
-        int rc = get_field(ctx, PD_PF_C, 1, c);
-        if (!rc) rc = get_field(ctx, PD_PF_H, 1, H);
-        if (!rc) rc = get_field(ctx, PD_PF_FP, 1, pf_Fp);
-        if (!rc) rc = get_field(ctx, PD_PF_VOL, 1, vol);
-        return rc;
+        const FieldOut out[4] = { { ctx->pdf(PD_PF_C), 1, sizeof(double), c }, { ctx->pdf(PD_PF_H), 1, sizeof(double), H },
+            { ctx->pdf(PD_PF_FP), 1, sizeof(double), pf_Fp }, { ctx->pdf(PD_PF_VOL), 1, sizeof(double), vol } };
+        return read_fields(ctx, out, 4);
     }
     // the solve's own fields are not on the device: their host values stand
     int rc = download(ctx);
@@ -945,7 +988,7 @@ int zmpm_get_viscoelastic_strain(zmpm_ctx* ctx, double* Fe)
 {
     if (!ctx || !Fe) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
-    if (ctx->uploaded && ctx->pd_active == PD_FIELDS) return get_field(ctx, PD_FE, 9, Fe);
+    if (ctx->uploaded && ctx->pd_active == PD_FIELDS) return read_field(ctx, PD_FE, 9, Fe);
     std::memcpy(Fe, ctx->hFe.data(), 9 * ctx->P * sizeof(double));
     return ZMPM_OK;
 }
@@ -1036,8 +1079,8 @@ int zmpm_get_plastic_state(zmpm_ctx* ctx, double* ys, int32_t* broken)
     if (!ctx) return ZMPM_BAD_ARG;
     cudaSetDevice(ctx->device);
     if (ctx->uploaded) {
-        int rc = get_field(ctx, PD_YS, 1, ys);
-        return rc ? rc : get_field(ctx, PI_BROKEN, broken);
+        const FieldOut out[2] = { { ctx->pdf(PD_YS), 1, sizeof(double), ys }, { ctx->pif(PI_BROKEN), 1, sizeof(int32_t), broken } };
+        return read_fields(ctx, out, 2);
     }
     for (int64_t i = 0; i < ctx->P; ++i) {
         if (ys) ys[i] = ctx->hys[i];
@@ -1411,7 +1454,7 @@ int zmpm_adjoint_substep(zmpm_ctx* ctx, double dt, const zmpm_solver* s, double 
             k_fields_to_host<<<(unsigned)((P + 255) / 256), 256, 0, sm>>>(stg + off, nc[a], P, cap, ctx->slot_of_id.as<int32_t>(),
                 aj + (int64_t)fld[a] * cap);
             ++g_kernel_launches;
-            ZMPM_CUDA(copy_out(ctx, dst[a], stg + off, nc[a] * P * sizeof(double)));
+            ZMPM_CUDA(cudaMemcpyAsync(dst[a], stg + off, nc[a] * P * sizeof(double), cudaMemcpyDeviceToHost, sm));
             off += nc[a] * P;
         }
         if (gE) {
