@@ -457,12 +457,15 @@ struct RowsScatter {
     }
 };
 
-// Affine: item (component, cell) adds w_ip (q + a i + b j + c k), a vector
-// written affinely in the node offset (i, j, k).  MASS (APIC P2G,
-// particlesToGridHelper, MpmSimulationBase.cpp:563-608): component 0 adds w_ip
-// m_p and components 1-3 the momentum m (v + C (x_i - x_p)); without it the
-// three components are a vector (the MLS-MPM force).  Records: fractions at
-// 0-2, the mass at 3 if any, then (q, a, b, c) of each vector component.
+// Affine: item (component, cell) adds w_ip (q + a (i - 1) + b (j - 1) + c (k - 1)),
+// a vector written affinely in the node offset from the stencil's centre, which
+// lies within half a cell of the particle: no term is larger than the vector at
+// the stencil's nodes (about node 0 the terms were up to twice as large, and the
+// FP32 MLS-MPM force lost up to 5%).  MASS (APIC P2G, particlesToGridHelper,
+// MpmSimulationBase.cpp:563-608): component 0 adds w_ip m_p and components 1-3 the
+// momentum m (v + C (x_i - x_p)); without it the three components are a vector
+// (the MLS-MPM force).  Records: fractions at 0-2, the mass at 3 if any, then (q,
+// a, b, c) of each vector component.
 template <class T, bool MASS>
 struct AffineScatter {
     static constexpr int NF = MASS ? 16 : 15, NC = MASS ? 4 : 3;
@@ -489,20 +492,20 @@ struct AffineScatter {
                     by = f2(row[2 * FS + p], sq * row[2 * FS + pq]);
                     cz = f2(row[3 * FS + p], sq * row[3 * FS + pq]);
                 }
-                const float2 wx1 = w[0][1], wx2 = mul2(w[0][2], f2(2.f)); // i w_i for i = 1, 2
+                const float2 nw0 = mul2(w[0][0], f2(-1.f)); // (i - 1) w_i: -w_0, 0, w_2
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const float2 t = mul2(w[1][j], w[2][k]);
-                        // (q + b j + c k) t and a t
+                        // (q + b (j - 1) + c (k - 1)) t and a t
                         float2 l = q0;
-                        if (j) l = fma2(by, f2((float)j), l);
-                        if (k) l = fma2(cz, f2((float)k), l);
+                        if (j != 1) l = fma2(by, f2((float)(j - 1)), l);
+                        if (k != 1) l = fma2(cz, f2((float)(k - 1)), l);
                         const float2 u = mul2(l, t), v = mul2(ax, t);
-                        a2[3 * j + k] = fma2(w[0][0], u, a2[3 * j + k]);
-                        a2[9 + 3 * j + k] = fma2(w[0][1], u, fma2(wx1, v, a2[9 + 3 * j + k]));
-                        a2[18 + 3 * j + k] = fma2(w[0][2], u, fma2(wx2, v, a2[18 + 3 * j + k]));
+                        a2[3 * j + k] = fma2(w[0][0], u, fma2(nw0, v, a2[3 * j + k]));
+                        a2[9 + 3 * j + k] = fma2(w[0][1], u, a2[9 + 3 * j + k]);
+                        a2[18 + 3 * j + k] = fma2(w[0][2], u, fma2(w[0][2], v, a2[18 + 3 * j + k]));
                     }
             }
 #pragma unroll
@@ -522,9 +525,9 @@ struct AffineScatter {
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const T t = w[1][j] * w[2][k];
-                        const T u = (q0 + by * T(j) + cz * T(k)) * t, v = ax * t;
+                        const T u = (q0 + by * T(j - 1) + cz * T(k - 1)) * t, v = ax * t;
 #pragma unroll
-                        for (int i = 0; i < 3; ++i) a[9 * i + 3 * j + k] += w[0][i] * u + (T(i) * w[0][i]) * v;
+                        for (int i = 0; i < 3; ++i) a[9 * i + 3 * j + k] += w[0][i] * (u + T(i - 1) * v);
                     }
             }
         }

@@ -56,7 +56,7 @@ struct P2gPhase1 {
 #pragma unroll
             for (int q = 0; q < 3; ++q) mC[q] = (T)(mass * pd[(PD_C + 3 * r + q) * cap + s]);
             const T mv = (T)(mass * pd[(PD_V + r) * cap + s]);
-            rc[(4 + 4 * r) * FS] = mv - tdx * (mC[0] * fr[0] + mC[1] * fr[1] + mC[2] * fr[2]);
+            rc[(4 + 4 * r) * FS] = mv + tdx * (mC[0] * (T(1) - fr[0]) + mC[1] * (T(1) - fr[1]) + mC[2] * (T(1) - fr[2]));
 #pragma unroll
             for (int q = 0; q < 3; ++q) rc[(5 + 4 * r + q) * FS] = tdx * mC[q];
         }
@@ -182,7 +182,7 @@ __device__ __forceinline__ void force_record(const M3<T>& S, const T fr[3], T in
         const T k = T(-4) * inv_dx; // dx D^-1
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            rc[(3 + 4 * r) * FS] = -k * (S(r, 0) * fr[0] + S(r, 1) * fr[1] + S(r, 2) * fr[2]);
+            rc[(3 + 4 * r) * FS] = k * (S(r, 0) * (T(1) - fr[0]) + S(r, 1) * (T(1) - fr[1]) + S(r, 2) * (T(1) - fr[2]));
 #pragma unroll
             for (int c = 0; c < 3; ++c) rc[(4 + 4 * r + c) * FS] = k * S(r, c);
         }
