@@ -33,7 +33,7 @@ def test_group_sizes(cuda_lib, oracle, n, spread, precision):
     assert_bins_equal(g.binParticles(), b)  # from sorted slots
 
 
-# groups around the 16384 that are ranked pairwise, one or two particles each
+# thousands of groups more than are ranked pairwise, one or two particles each
 @pytest.mark.parametrize("extra", [-1, 0, 1])
 def test_group_counts(cuda_lib, oracle, extra):
     g = np.stack(np.meshgrid(np.arange(32), np.arange(32), np.arange(17), indexing="ij"), -1).reshape(-1, 3)
@@ -63,3 +63,39 @@ def test_tables_stay_clean(cuda_lib, oracle):
         o = mpm.MpmSimulation(DX, precision="fp64", lib=oracle)
         o.addParticles(x, None, 1.0, 1.0)
         assert_bins_equal(g.binParticles(), o.binParticles())
+
+
+# groups around the 8192 that are ranked pairwise, and a large group: a context takes the way of its last scene and
+# finds back to the other
+@pytest.mark.parametrize("groups", [8191, 8192, 8193])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_group_limit_and_way_back(cuda_lib, oracle, groups, precision):
+    page = np.array([2, 4, 4] if precision == "fp64" else [4, 4, 4])
+    g = np.stack(np.meshgrid(np.arange(20), np.arange(20), np.arange(21), indexing="ij"), -1).reshape(-1, 3)
+    rng = np.random.default_rng(11)
+    many = page * g[rng.permutation(len(g))[:groups]] + 8 + 0.6 + (page - 1.2) * rng.random((groups, 3))
+    few = 40 + 8 * rng.random((groups, 3))
+    few[2200:] += 30 * rng.random((groups - 2200, 3))
+    cell = 40.55 + 0.9 * rng.random((groups, 3))  # one group of all
+    s = mpm.MpmSimulation(1.0 / 256, precision=precision, grid_log2=8)
+    s.addParticles(many / 256, None, 1.0, 1.0)
+    for x in (many, few, cell, many, cell, few, few, many):
+        x = (x / 256).astype(np.float32).astype(np.float64)
+        s.setParticles(X=x)
+        o = mpm.MpmSimulation(1.0 / 256, precision=precision, lib=oracle)
+        o.addParticles(x, None, 1.0, 1.0)
+        for _ in range(2):
+            assert_bins_equal(s.binParticles(), o.binParticles())
+
+
+def test_large_scenes_count_their_pages_once(cuda_lib):
+    """A scene for the radix way is not put through the page counts again on every pass."""
+    rng = np.random.default_rng(5)
+    s = mpm.MpmSimulation(DX, precision="fp64", grid_log2=7)
+    s.addParticles((32.55 + 0.9 * rng.random((4000, 3))) * DX, None, 1.0, 1.0)
+    s.useExplicit()
+    n = []
+    for _ in range(3):
+        assert s.advanceOneTimeStep(1e-4) == abi.OK
+        n.append(s.last_stats["kernel_launches"])
+    assert n[1] == n[2] == n[0] - 3  # the counts, the pages, the unmarking

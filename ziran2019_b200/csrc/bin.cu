@@ -23,8 +23,10 @@
 // more than RANK_MAX groups (pairwise comparison grows quadratically) or with a
 // group of more than ORDER_CAP particles (shared memory, and one cell may hold
 // them all) take the radix sort over particle keys of steps 1-4 above: about 40
-// launches.  Measured at 60k particles in FP64 the radix way's kernels took 0.19
-// of a 0.37 ms explicit substep.
+// launches.  A context stays on the radix way until a pass on it finds a scene
+// for the other (counting the pages first cost such scenes 0.06 ms a pass).
+// Measured at 60k particles in FP64 the radix way's kernels took 0.19 of a 0.37 ms
+// explicit substep.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -187,8 +189,14 @@ __global__ void k_group_nbr(const int4* __restrict__ group_page, int64_t G, Page
 }
 
 // ------------------------------------------------------ binning by page ----
-constexpr int RANK_MAX = 16384;       // groups: 2^28 comparisons
-constexpr int ORDER_CAP = 2048;       // particles of one group: 32 KB of shared memory
+// Groups up to which comparing all pairs (k_rank) is worth it.  A pass by page
+// and by radix sort, 2 particles per group: 5000 groups 0.122 ms by page, 7000
+// 0.214 and 0.231, 8000 0.258 and 0.226, 16000 0.545 and 0.267; 128 per group: 7000
+// 0.325 and 0.38, 8000 0.383 and 0.40, 16000 0.79 and 0.59.  In a substep, where the
+// radix way's 30 launches more also leave gaps, the two meet between 8400 and
+// 10700 groups.
+constexpr int RANK_MAX = 8192;
+constexpr int ORDER_CAP = 2048;       // particles of one group: 16 KB of shared memory
 constexpr int32_t MARK = 0x70000000;  // first-touch table: a page of this pass, above any emission, below the clean values
 
 // Base node of every slot, particles per page; the particle that finds its
@@ -359,20 +367,35 @@ __global__ void __launch_bounds__(BIN_THREADS) k_order(const int32_t* __restrict
 // The cell records of sorted groups (the radix way): one warp per group, cell
 // starts by the heads of equal elements.
 template <class L>
-__global__ void __launch_bounds__(32) k_cells(const int32_t* __restrict__ group_start, const short4* __restrict__ base, int32_t* __restrict__ cells)
+__global__ void __launch_bounds__(32) k_cells(const int32_t* __restrict__ group_start, const short4* __restrict__ base, int32_t* __restrict__ cells,
+    DevCounters* __restrict__ dc)
 {
     __shared__ int32_t start[L::NPB + 1];
     const int g = blockIdx.x, lane = threadIdx.x, s0 = group_start[g], n = group_start[g + 1] - s0;
+    if (lane == 0) atomicMax(&dc->max_group, n);
     for (int e = lane; e <= L::NPB; e += 32) start[e] = n;
     __syncwarp();
+#pragma unroll 4
     for (int i = lane; i < n; i += 32) {
         const short4 b = base[s0 + i];
         const int e = (int)L::elem(b.x & (L::BX - 1), b.y & (L::BY - 1), b.z & (L::BZ - 1));
         atomicMin(&start[e], i);
     }
     __syncwarp();
-    if (lane == 0) // an empty cell starts where the next one does
-        for (int e = L::NPB - 1; e >= 0; --e) start[e] = start[e] < start[e + 1] ? start[e] : start[e + 1];
+    // an empty cell starts where the next one does: the smallest start from each cell on
+    constexpr int PER = L::NPB / 32;
+    int c[PER], m = n;
+#pragma unroll
+    for (int k = PER - 1; k >= 0; --k) {
+        m = min(m, start[lane * PER + k]);
+        c[k] = m;
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) m = min(m, __shfl_down_sync(0xffffffffu, m, o)); // of this lane's cells and all after
+    int after = __shfl_down_sync(0xffffffffu, m, 1);
+    if (lane == 31) after = n;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) start[lane * PER + k] = min(c[k], after);
     __syncwarp();
     write_cells<L>(start, g, cells);
 }
@@ -482,7 +505,7 @@ static int binning_radix(Ctx* ctx)
 
     ZMPM_CUDA(ctx->group_nbr.ensure(8 * G * sizeof(int32_t)));
     ZMPM_CUDA(ctx->group_cells.ensure(G * GroupCells<L>::WORDS * sizeof(int32_t)));
-    k_cells<L><<<(unsigned)G, 32, 0, st>>>(ctx->group_start.as<int32_t>(), ctx->base.as<short4>(), ctx->group_cells.as<int32_t>());
+    k_cells<L><<<(unsigned)G, 32, 0, st>>>(ctx->group_start.as<int32_t>(), ctx->base.as<short4>(), ctx->group_cells.as<int32_t>(), dc);
     ++g_kernel_launches;
     ZMPM_CUDA(ctx->emit_flag.ensure(8 * G * sizeof(int32_t)));
     ZMPM_CUDA(ctx->emit_scan.ensure(8 * G * sizeof(int32_t)));
@@ -495,9 +518,11 @@ static int binning_radix(Ctx* ctx)
     exclusive_scan<int32_t>(ctx->emit_flag.as<int32_t>(), ctx->emit_scan.as<int32_t>(), 8 * G, tot, sscr, st);
     int32_t hB = 0;
     ZMPM_CUDA(cudaMemcpyAsync(&hB, tot, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    ZMPM_CUDA(cudaMemcpyAsync(&ctx->hcounters, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
     ZMPM_CUDA(cudaStreamSynchronize(st));
     const int64_t B = hB;
     ctx->B = B;
+    ctx->bin_radix = G > RANK_MAX || ctx->hcounters.max_group > ORDER_CAP;
     ZMPM_CUDA(ctx->block_page.ensure(B * sizeof(int4)));
     ZMPM_CUDA(ctx->block_index.ensure(B * sizeof(uint64_t)));
     k_blocks<L><<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->emit_flag.as<int32_t>(), ctx->emit_scan.as<int32_t>(),
@@ -545,6 +570,7 @@ static int binning_impl(Ctx* ctx)
         ZMPM_CUDA(cudaMemsetAsync(first, 0x7f, ctx->table_size * sizeof(int32_t), st));
     }
     ctx->tables_dirty = true;
+    if (ctx->bin_radix) return binning_radix<L, KT>(ctx);
     k_count<L, KT><<<nblk(P), BIN_THREADS, 0, st>>>(ctx->pdf(PD_X), cap, P, 1.0 / ctx->cfg.dx, 1.0f / (float)ctx->cfg.dx, base_old, cnt, list,
         pdims, dc);
     k_pages<<<std::min(nblk(8 * P), 1024u), BIN_THREADS, 0, st>>>(list, pdims, cnt, list_cnt, first, dc);
@@ -563,6 +589,7 @@ static int binning_impl(Ctx* ctx)
             return ZMPM_OUT_OF_GRID;
         }
         ZMPM_CUDA(cudaMemsetAsync(dc, 0, sizeof(DevCounters), st));
+        ctx->bin_radix = true;
         return binning_radix<L, KT>(ctx);
     }
     ctx->G = G;

@@ -196,6 +196,7 @@ struct Ctx {
     DBuf group_start, group_page, group_nbr, emit_flag, emit_scan;
     DBuf group_cells;                     // GroupCells record per group (xfer.cuh)
     DBuf page_first, page_block, page_count; // dense page tables
+    bool bin_radix = false;               // the last binning pass was one for the radix way (bin.cu)
     bool tables_dirty = false;            // a binning pass that failed may have left marks in page_first and page_count
     DBuf page_list;                       // occupied pages in any order, then their particle counts (binning)
     DBuf block_page, block_index;         // per page: packed coords, page index
