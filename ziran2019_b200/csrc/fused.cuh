@@ -534,8 +534,14 @@ struct AffineScatter {
     }
 };
 
+// Occupied cells of a group below which its warps share the particles instead of
+// the cells: whole cells left three warps idle on a group of one.  Newton substep
+// of 1500 groups of 500 particles in 1 / 2 / 4 cells, FP32: 3.36, 2.86 and 2.67 ->
+// 2.15, 2.12 and 2.09 ms; FP64: 4.74, 4.36 and 4.01 -> 3.11, 3.07 and 3.01.
+constexpr int CUT_CELLS = 8;
+
 // One warp's part of a piece: the occupied cells whose first particle falls in
-// its quarter of the piece's particles.  Warps do not wait for one another
+// its quarter of the piece's particles (CUT_CELLS: the quarter itself).  Warps do not wait for one another
 // inside a piece; each alternates phase 1 (lane per particle, record into the
 // warp's own shared memory) and phase 2 (lane per (row, cell) item, one shared
 // atomic per node) over its own particles, so one warp's loads overlap
@@ -552,22 +558,33 @@ __device__ __forceinline__ void group_warp(GroupSmem<L, T, TX, Scatter::NF, Scat
     const uint8_t* occ = reinterpret_cast<const uint8_t*>(st + GroupCells<L>::OCC);
     const int a0 = pc.s0 - pc.g0, a1 = pc.s1 - pc.g0, n = a1 - a0;
     const int t0 = a0 + n * warp / FUSED_WARPS, t1 = a0 + n * (warp + 1) / FUSED_WARPS;
-    // the warp's run [lo, hi) of the occupied cells, by their first particle in the piece
-    int lo = 0, hi = 0;
-#pragma unroll
-    for (int k = 0; k < NPB; k += 32) {
-        bool below0 = false, below1 = false;
-        if (k + lane < nocc) {
-            const int c = occ[k + lane], b = st[c], e = st[c + 1], f = b > a0 ? b : a0;
-            below0 = e <= a0 || f < t0;
-            below1 = e <= a0 || f < t1;
-        }
-        lo += __popc(__ballot_sync(0xffffffffu, below0));
-        hi += __popc(__ballot_sync(0xffffffffu, below1));
+    // the warp's run [lo, hi) of the occupied cells and its particles [p_lo, p_hi)
+    int lo = 0, hi = 0, p_lo, p_hi;
+    if (nocc < CUT_CELLS) { // its quarter of the particles and the cells they lie in
+        if (t0 >= t1) return;
+        const int c = lane < nocc ? occ[lane] : 0;
+        lo = __popc(__ballot_sync(0xffffffffu, lane < nocc && st[c + 1] <= t0));
+        hi = __popc(__ballot_sync(0xffffffffu, lane < nocc && st[c] < t1));
+        p_lo = t0;
+        p_hi = t1;
     }
-    if (lo >= hi) return;
-    const int b0 = st[occ[lo]], e1 = st[occ[hi - 1] + 1];
-    const int p_lo = b0 > a0 ? b0 : a0, p_hi = e1 < a1 ? e1 : a1;
+    else { // the cells whose first particle in the piece falls in its quarter
+#pragma unroll
+        for (int k = 0; k < NPB; k += 32) {
+            bool below0 = false, below1 = false;
+            if (k + lane < nocc) {
+                const int c = occ[k + lane], b = st[c], e = st[c + 1], f = b > a0 ? b : a0;
+                below0 = e <= a0 || f < t0;
+                below1 = e <= a0 || f < t1;
+            }
+            lo += __popc(__ballot_sync(0xffffffffu, below0));
+            hi += __popc(__ballot_sync(0xffffffffu, below1));
+        }
+        if (lo >= hi) return;
+        const int b0 = st[occ[lo]], e1 = st[occ[hi - 1] + 1];
+        p_lo = b0 > a0 ? b0 : a0;
+        p_hi = e1 < a1 ? e1 : a1;
+    }
     T* rec = sm.rec[warp];
     double* acc = sm.acc[SM::ACCS == 2 ? ph & 1 : 0];
     const int ncell = hi - lo, items = NC * ncell;
