@@ -44,7 +44,7 @@ def launches(x, precision, layout, iters):
 
 
 def expected(x, precision, layout):
-    """The rule: the stencil where its bytes are at most 1 KB per particle, a group counting as 192 particles."""
+    """The rule below 96 MB: the stencil where its bytes are at most 1 KB per particle, a group counting as 192."""
     page = np.array([2 if layout == "244" else 4, 4, 4])
     groups = np.unique(np.floor(x / DX - 0.5).astype(int) // page, axis=0)
     near = np.stack(np.meshgrid(*[np.arange(2)] * 3, indexing="ij"), -1).reshape(-1, 3)

@@ -375,15 +375,24 @@ __global__ void __launch_bounds__(FUSED_THREADS, 4) k_mr_stencil(NodeGeom ng, in
 }
 
 // -------------------------------------------------------------- host side --
-// The stencil costs its coefficient reads per page (0.2 ns per KB measured
-// from L2 and HBM), the matrix-free product 0.19 ns per particle and about 192
-// particles' worth per group: the stencil is taken where its bytes are below
-// 1 KB per such unit (dense scenes need about 150 B; a spray of single
-// particles, 500 KB each, stays matrix-free).
+// The stencil's product costs the reads of its coefficients, the matrix-free one
+// its particles and about 192 particles' worth per group; the rule is a limit of
+// bytes per such unit (a dense scene has about 150, a spray of single particles
+// up to 2600).  Coefficients that stay in L2 win at any density measured; above
+// that sparse scenes lose.  Substeps of four iterations with 20 products each,
+// matrix-free / stencil, against MB of coefficients and bytes per unit:
+//   FP64  43.5, 665: 3.13 / 2.35 ms;  104, 625: 4.15 / 4.33;  168, 629: 5.7 / 7.1;
+//         215, 216: 12.0 / 11.4;  202, 321: 8.5 / 9.4;  182, 489: 6.3 / 7.8
+//   FP32  99.6, 426: 5.9 / 5.3;  164, 368: 8.0 / 8.3;  319, 345: 16.1 / 15.6;
+//         108, 247: 7.5 / 6.5;  287, 201: 22.0 / 17.2
+// Few iterations do not change the side: the assembly costs less than the gathers
+// it saves in the preconditioner (498k particles, one iteration of 3 products: 5.7
+// / 2.7 ms).
 bool stencil_pays(const Ctx* ctx)
 {
     const double bytes = (double)ctx->B * STENCIL * ctx->npb() * (ctx->mixed ? sizeof(float) : sizeof(double));
-    return bytes <= 1024.0 * ((double)ctx->P + 192.0 * (double)ctx->G);
+    const double units = (double)ctx->P + 192.0 * (double)ctx->G;
+    return bytes <= (bytes <= 96e6 ? 1024.0 : (ctx->mixed ? 352.0 : 256.0)) * units;
 }
 
 template <class L, class T>
