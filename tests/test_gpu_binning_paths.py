@@ -99,3 +99,15 @@ def test_large_scenes_count_their_pages_once(cuda_lib):
         assert s.advanceOneTimeStep(1e-4) == abi.OK
         n.append(s.last_stats["kernel_launches"])
     assert n[1] == n[2] == n[0] - 3  # the counts, the pages, the unmarking
+
+
+@pytest.mark.parametrize("precision,nodes_per_page", [("fp64", 32), ("mixed", 64)])
+def test_two_page_tables(cuda_lib, precision, nodes_per_page):
+    """A context holds two words per page of the grid, not more (the tables are 8.6 GB each at grid_log2 = 12, FP64)."""
+    import torch
+    table = 4 * (1 << 30) // nodes_per_page
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    s = mpm.MpmSimulation(DX, precision=precision, grid_log2=10)
+    assert free - torch.cuda.mem_get_info()[0] < 2.8 * table + (8 << 20)  # with the rounding up of allocations
+    s.close()

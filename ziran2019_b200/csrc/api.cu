@@ -606,8 +606,6 @@ int zmpm_create(const zmpm_config* cfg, zmpm_ctx** out)
     ctx->table_size = (int64_t)ctx->pages[0] * ctx->pages[1] * ctx->pages[2];
     if ((e = ctx->page_first.ensure(ctx->table_size * sizeof(int32_t))) != cudaSuccess) return fail(e);
     if ((e = ctx->page_block.ensure(ctx->table_size * sizeof(int32_t))) != cudaSuccess) return fail(e);
-    if ((e = ctx->page_count.ensure(ctx->table_size * sizeof(int32_t))) != cudaSuccess) return fail(e);
-    if ((e = cudaMemset(ctx->page_count.p, 0, ctx->table_size * sizeof(int32_t))) != cudaSuccess) return fail(e);
     if ((e = cudaMemset(ctx->page_first.p, 0x7f, ctx->table_size * sizeof(int32_t))) != cudaSuccess) return fail(e);
     if ((e = ctx->counters.ensure(sizeof(DevCounters))) != cudaSuccess) return fail(e);
     if ((e = ctx->scal.ensure(sizeof(SolverScalars))) != cudaSuccess) return fail(e);
@@ -630,7 +628,7 @@ int zmpm_destroy(zmpm_ctx* ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DBuf* bufs[] = { &ctx->pd, &ctx->pd_alt, &ctx->pi, &ctx->pi_alt, &ctx->slot_of_id, &ctx->base_by_id, &ctx->base, &ctx->Fn, &ctx->scratch,
         &ctx->frac, &ctx->stress, &ctx->keys, &ctx->keys_alt, &ctx->flags_i32, &ctx->scan_i32, &ctx->scan_scr, &ctx->radix_scr, &ctx->group_start,
-        &ctx->group_page, &ctx->group_nbr, &ctx->emit_flag, &ctx->emit_scan, &ctx->page_first, &ctx->page_block, &ctx->page_count, &ctx->page_list,
+        &ctx->group_page, &ctx->group_nbr, &ctx->emit_flag, &ctx->emit_scan, &ctx->page_first, &ctx->page_block, &ctx->page_list,
         &ctx->group_cells, &ctx->block_page,
         &ctx->block_index, &ctx->gm, &ctx->gmv, &ctx->vn, &ctx->dv, &ctx->vstar, &ctx->facc, &ctx->res, &ctx->proj, &ctx->collided,
         &ctx->node_idx, &ctx->red, &ctx->scal, &ctx->counters, &ctx->dcolliders, &ctx->adm_F, &ctx->adm_gvn, &ctx->adm_B, &ctx->adm_pre,

@@ -54,6 +54,14 @@ struct PageDims {
     __device__ __forceinline__ int64_t index(int x, int y, int z) const { return ((int64_t)x * py + y) * pz + z; }
 };
 
+// The dense page table.  Between passes every word is PAGE_CLEAN.  Binning by page
+// subtracts the page's particles (fewer than 2^27, so PAGE_BIT stays set), clears
+// PAGE_BIT in every page that gets a block and puts PAGE_CURSOR plus the next free
+// slot into the groups' pages; both ways then take the smallest emission that touches
+// the page, which is below all of these (below 8 RANK_MAX by page; below 2^30 by
+// radix sort, which starts from clean words).
+constexpr int32_t PAGE_CLEAN = 0x7f7f7f7f, PAGE_BIT = 0x40000000, PAGE_CURSOR = 0x40000000;
+
 // Base node of the particle in slot s, or node 0 and false when its stencil
 // leaves the grid.  KT: precision of the key arithmetic (double for FP64 runs, float for the
 // mixed runs whose grid mirrors the reference's T=float build).
@@ -176,7 +184,7 @@ __global__ void k_blocks(const int4* __restrict__ group_page, int64_t G, PageDim
 }
 
 __global__ void k_group_nbr(const int4* __restrict__ group_page, int64_t G, PageDims pd, const int32_t* __restrict__ page_block,
-    int32_t* __restrict__ first, int32_t* __restrict__ nbr, int32_t* __restrict__ cnt)
+    int32_t* __restrict__ first, int32_t* __restrict__ nbr)
 {
     int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= 8 * G) return;
@@ -184,8 +192,7 @@ __global__ void k_group_nbr(const int4* __restrict__ group_page, int64_t G, Page
     int t = (int)(e & 7);
     int64_t idx = pd.index(gp.x + (t >> 2), gp.y + ((t >> 1) & 1), gp.z + (t & 1));
     nbr[e] = page_block[idx];
-    first[idx] = 0x7fffffff; // leave the first-touch table clean for the next pass
-    if (cnt && t == 0) cnt[idx] = 0; // and the page counters (t = 0 is the group's page)
+    first[idx] = PAGE_CLEAN; // for the next pass
 }
 
 // ------------------------------------------------------ binning by page ----
@@ -197,14 +204,13 @@ __global__ void k_group_nbr(const int4* __restrict__ group_page, int64_t G, Page
 // 10700 groups.
 constexpr int RANK_MAX = 8192;
 constexpr int ORDER_CAP = 2048;       // particles of one group: 16 KB of shared memory
-constexpr int32_t MARK = 0x70000000;  // first-touch table: a page of this pass, above any emission, below the clean values
 
 // Base node of every slot, particles per page; the particle that finds its
-// page's counter at zero appends the page to the list.  Slots are in the last
+// page clean appends the page to the list.  Slots are in the last
 // pass's order, so the lanes of a warp mostly share a page and count as one.
 template <class L, class KT>
 __global__ void __launch_bounds__(BIN_THREADS) k_count(const double* __restrict__ x, int64_t cap, int64_t P, double inv_dx_d, float inv_dx_f,
-    short4* __restrict__ base, int32_t* __restrict__ cnt, int4* __restrict__ list, PageDims pd, DevCounters* __restrict__ dc)
+    short4* __restrict__ base, int32_t* __restrict__ first, int4* __restrict__ list, PageDims pd, DevCounters* __restrict__ dc)
 {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = s < P;
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_count(const double* __restrict_
     const int64_t page = in ? pd.index(p0, p1, p2) : -1;
     const unsigned peers = __match_any_sync(0xffffffffu, page);
     if (!in || (threadIdx.x & 31) != __ffs(peers) - 1) return;
-    if (atomicAdd(&cnt[page], __popc(peers)) == 0) {
+    if (atomicSub(&first[page], __popc(peers)) == PAGE_CLEAN) {
         const unsigned long long g = atomicAdd(reinterpret_cast<unsigned long long*>(&dc->G), 1ull);
         list[g] = make_int4(p0, p1, p2, (int)(uint32_t)L::page_index(p0, p1, p2));
     }
@@ -225,41 +231,40 @@ __global__ void __launch_bounds__(BIN_THREADS) k_count(const double* __restrict_
 
 // Per listed page: its particle count, the largest count, and the number of
 // distinct pages among it and its 7 upper neighbours.
-__global__ void __launch_bounds__(BIN_THREADS) k_pages(const int4* __restrict__ list, PageDims pd, const int32_t* __restrict__ cnt,
-    int32_t* __restrict__ list_cnt, int32_t* __restrict__ first, DevCounters* __restrict__ dc)
+__global__ void __launch_bounds__(BIN_THREADS) k_pages(const int4* __restrict__ list, PageDims pd, int32_t* __restrict__ list_cnt,
+    int32_t* __restrict__ first, DevCounters* __restrict__ dc)
 {
     const int64_t G = dc->G;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < 8 * G; e += (int64_t)gridDim.x * blockDim.x) {
         const int4 p = list[e >> 3];
         const int t = (int)(e & 7);
         const int64_t idx = pd.index(p.x + (t >> 2), p.y + ((t >> 1) & 1), p.z + (t & 1));
-        if (atomicMin(&first[idx], MARK) > MARK) atomicAdd(reinterpret_cast<unsigned long long*>(&dc->B), 1ull);
+        const int32_t was = atomicAnd(&first[idx], ~PAGE_BIT);
+        if (was & PAGE_BIT) atomicAdd(reinterpret_cast<unsigned long long*>(&dc->B), 1ull);
         if (t == 0) {
-            const int c = cnt[idx];
+            const int c = PAGE_CLEAN - (was | PAGE_BIT);
             list_cnt[e >> 3] = c;
             atomicMax(&dc->max_group, c);
         }
     }
 }
 
-// Leaves both page tables clean when the pass stops after k_pages.
-__global__ void __launch_bounds__(BIN_THREADS) k_unmark(const int4* __restrict__ list, int64_t G, PageDims pd, int32_t* __restrict__ cnt,
-    int32_t* __restrict__ first)
+// Leaves the page table clean when the pass stops after k_pages.
+__global__ void __launch_bounds__(BIN_THREADS) k_unmark(const int4* __restrict__ list, int64_t G, PageDims pd, int32_t* __restrict__ first)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= 8 * G) return;
     const int4 p = list[e >> 3];
     const int t = (int)(e & 7);
     const int64_t idx = pd.index(p.x + (t >> 2), p.y + ((t >> 1) & 1), p.z + (t & 1));
-    first[idx] = 0x7fffffff;
-    if (t == 0) cnt[idx] = 0;
+    first[idx] = PAGE_CLEAN;
 }
 
 // One warp per listed page: its rank among the page indices and its first slot
-// (the particles of the smaller ones); the page's counter becomes the cursor of
+// (the particles of the smaller ones); the page's word becomes the cursor of
 // k_place.
 __global__ void __launch_bounds__(BIN_THREADS) k_rank(const int4* __restrict__ list, const int32_t* __restrict__ list_cnt, int G, int64_t P,
-    PageDims pd, int32_t* __restrict__ group_start, int4* __restrict__ group_page, int32_t* __restrict__ cnt)
+    PageDims pd, int32_t* __restrict__ group_start, int4* __restrict__ group_page, int32_t* __restrict__ first)
 {
     const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= G) return;
@@ -280,7 +285,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_rank(const int4* __restrict__ l
     if (lane != 0) return;
     group_start[rank] = start;
     group_page[rank] = make_int4(p.x, p.y, p.z, p.w);
-    cnt[pd.index(p.x, p.y, p.z)] = start;
+    first[pd.index(p.x, p.y, p.z)] = PAGE_CURSOR + start;
     if (i == 0) group_start[G] = (int32_t)P;
 }
 
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_rank(const int4* __restrict__ l
 // key above its old slot.
 template <class L>
 __global__ void __launch_bounds__(BIN_THREADS) k_place(const short4* __restrict__ base, int64_t P, const int32_t* __restrict__ orig_id,
-    PageDims pd, int32_t* __restrict__ cursor, uint64_t* __restrict__ pairs)
+    PageDims pd, int32_t* __restrict__ first, uint64_t* __restrict__ pairs)
 {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = s < P;
@@ -297,7 +302,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_place(const short4* __restrict_
     const unsigned peers = __match_any_sync(0xffffffffu, page);
     const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
     int at = 0;
-    if (in && lane == leader) at = atomicAdd(&cursor[page], __popc(peers));
+    if (in && lane == leader) at = atomicAdd(&first[page], __popc(peers)) - PAGE_CURSOR;
     at = __shfl_sync(0xffffffffu, at, leader);
     if (!in) return;
     at += __popc(peers & ((1u << lane) - 1u));
@@ -455,8 +460,8 @@ __global__ void __launch_bounds__(1024) k_number(const int4* __restrict__ group_
     }
 }
 
-// The radix way (see the top of the file); dc is zeroed and the page tables are
-// clean, but counted as dirty until the pass is complete.
+// The radix way (see the top of the file); dc is zeroed and the page table is
+// clean, but counts as dirty until the pass is complete.
 template <class L, class KT>
 static int binning_radix(Ctx* ctx)
 {
@@ -528,10 +533,10 @@ static int binning_radix(Ctx* ctx)
     k_blocks<L><<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->emit_flag.as<int32_t>(), ctx->emit_scan.as<int32_t>(),
         ctx->page_block.as<int32_t>(), ctx->block_page.as<int4>(), ctx->block_index.as<uint64_t>());
     ++g_kernel_launches;
-    k_group_nbr<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->page_block.as<int32_t>(), first, ctx->group_nbr.as<int32_t>(), nullptr);
+    k_group_nbr<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->page_block.as<int32_t>(), first, ctx->group_nbr.as<int32_t>());
     ++g_kernel_launches;
     ZMPM_CUDA(cudaGetLastError());
-    ctx->tables_dirty = false;
+    ctx->table_dirty = false;
     ctx->binned = true;
     return ZMPM_OK;
 }
@@ -559,32 +564,28 @@ static int binning_impl(Ctx* ctx)
 
     int4* list = ctx->page_list.as<int4>();
     int32_t* list_cnt = reinterpret_cast<int32_t*>(list + P);
-    int32_t* cnt = ctx->page_count.as<int32_t>();
     int32_t* first = ctx->page_first.as<int32_t>();
     short4* base_old = ctx->base_by_id.as<short4>(); // here by old slot
-    // A pass marks both page tables and clears the marks at its end; one that
-    // stopped in between (a failed allocation) left them, and a pass over such
-    // tables would miss pages and place particles out of range.
-    if (ctx->tables_dirty) {
-        ZMPM_CUDA(cudaMemsetAsync(cnt, 0, ctx->table_size * sizeof(int32_t), st));
-        ZMPM_CUDA(cudaMemsetAsync(first, 0x7f, ctx->table_size * sizeof(int32_t), st));
-    }
-    ctx->tables_dirty = true;
+    // A pass marks the page table and clears the marks at its end; one that
+    // stopped in between (a failed allocation) left them, and a pass over such a
+    // table would miss pages and place particles out of range.
+    if (ctx->table_dirty) ZMPM_CUDA(cudaMemsetAsync(first, PAGE_CLEAN & 0xff, ctx->table_size * sizeof(int32_t), st));
+    ctx->table_dirty = true;
     if (ctx->bin_radix) return binning_radix<L, KT>(ctx);
-    k_count<L, KT><<<nblk(P), BIN_THREADS, 0, st>>>(ctx->pdf(PD_X), cap, P, 1.0 / ctx->cfg.dx, 1.0f / (float)ctx->cfg.dx, base_old, cnt, list,
+    k_count<L, KT><<<nblk(P), BIN_THREADS, 0, st>>>(ctx->pdf(PD_X), cap, P, 1.0 / ctx->cfg.dx, 1.0f / (float)ctx->cfg.dx, base_old, first, list,
         pdims, dc);
-    k_pages<<<std::min(nblk(8 * P), 1024u), BIN_THREADS, 0, st>>>(list, pdims, cnt, list_cnt, first, dc);
+    k_pages<<<std::min(nblk(8 * P), 1024u), BIN_THREADS, 0, st>>>(list, pdims, list_cnt, first, dc);
     g_kernel_launches += 2;
     ZMPM_CUDA(cudaMemcpyAsync(&ctx->hcounters, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
     ZMPM_CUDA(cudaStreamSynchronize(st));
     const int64_t G = ctx->hcounters.G, B = ctx->hcounters.B;
     const bool out = (ctx->hcounters.flags & FLAG_OUT_OF_GRID) != 0;
     if (out || G > RANK_MAX || ctx->hcounters.max_group > ORDER_CAP) {
-        k_unmark<<<nblk(8 * G), BIN_THREADS, 0, st>>>(list, G, pdims, cnt, first);
+        k_unmark<<<nblk(8 * G), BIN_THREADS, 0, st>>>(list, G, pdims, first);
         ++g_kernel_launches;
         ZMPM_CUDA(cudaGetLastError());
         if (out) {
-            ctx->tables_dirty = false;
+            ctx->table_dirty = false;
             ctx->err = "a particle's stencil leaves the grid (raise grid_log2 or move the scene)";
             return ZMPM_OUT_OF_GRID;
         }
@@ -601,8 +602,8 @@ static int binning_impl(Ctx* ctx)
     int32_t* gstart = ctx->group_start.as<int32_t>();
     int4* gpage = ctx->group_page.as<int4>();
     int32_t* old_slot = ctx->flags_i32.as<int32_t>();
-    k_rank<<<nblk(32 * G), BIN_THREADS, 0, st>>>(list, list_cnt, (int)G, P, pdims, gstart, gpage, cnt);
-    k_place<L><<<nblk(P), BIN_THREADS, 0, st>>>(base_old, P, ctx->pif(PI_ID), pdims, cnt, ctx->keys_alt.as<uint64_t>());
+    k_rank<<<nblk(32 * G), BIN_THREADS, 0, st>>>(list, list_cnt, (int)G, P, pdims, gstart, gpage, first);
+    k_place<L><<<nblk(P), BIN_THREADS, 0, st>>>(base_old, P, ctx->pif(PI_ID), pdims, first, ctx->keys_alt.as<uint64_t>());
     k_order<L><<<(unsigned)G, BIN_THREADS, 0, st>>>(gstart, gpage, ctx->keys_alt.as<uint64_t>(), ctx->keys.as<uint64_t>(), old_slot,
         ctx->base.as<short4>(), ctx->group_cells.as<int32_t>());
     k_move<L><<<nblk(P), BIN_THREADS, 0, st>>>(ctx->keys.as<uint64_t>(), old_slot, P, cap, ctx->pd_active, ctx->pd.as<double>(),
@@ -612,10 +613,10 @@ static int binning_impl(Ctx* ctx)
     k_emit<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, first);
     k_number<L><<<1, 1024, 0, st>>>(gpage, (int)G, pdims, first, ctx->page_block.as<int32_t>(), ctx->block_page.as<int4>(),
         ctx->block_index.as<uint64_t>());
-    k_group_nbr<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->page_block.as<int32_t>(), first, ctx->group_nbr.as<int32_t>(), cnt);
+    k_group_nbr<<<nblk(8 * G), BIN_THREADS, 0, st>>>(gpage, G, pdims, ctx->page_block.as<int32_t>(), first, ctx->group_nbr.as<int32_t>());
     g_kernel_launches += 7;
     ZMPM_CUDA(cudaGetLastError());
-    ctx->tables_dirty = false;
+    ctx->table_dirty = false;
     ctx->binned = true;
     return ZMPM_OK;
 }

@@ -195,9 +195,9 @@ struct Ctx {
     DBuf keys, keys_alt, flags_i32, scan_i32, scan_scr, radix_scr;
     DBuf group_start, group_page, group_nbr, emit_flag, emit_scan;
     DBuf group_cells;                     // GroupCells record per group (xfer.cuh)
-    DBuf page_first, page_block, page_count; // dense page tables
+    DBuf page_first, page_block; // dense page tables
     bool bin_radix = false;               // the last binning pass was one for the radix way (bin.cu)
-    bool tables_dirty = false;            // a binning pass that failed may have left marks in page_first and page_count
+    bool table_dirty = false;             // a binning pass that failed may have left marks in page_first
     DBuf page_list;                       // occupied pages in any order, then their particle counts (binning)
     DBuf block_page, block_index;         // per page: packed coords, page index
     int64_t G = 0, B = 0, N = 0;
