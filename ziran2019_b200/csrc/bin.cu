@@ -20,7 +20,7 @@
 // from comparing their page indices pairwise, and each group's particles are
 // ordered in shared memory by one CTA (k_count, k_pages, one host read of the
 // counts, k_rank, k_place, k_order, k_emit, k_number): 9 launches.  Scenes with
-// more than RANK_MAX groups (pairwise comparison grows quadratically) or with a
+// more than RANK_MAX groups (see there) or with a
 // group of more than ORDER_CAP particles (shared memory, and one cell may hold
 // them all) take the radix sort over particle keys of steps 1-4 above: about 40
 // launches.  A context stays on the radix way until a pass on it finds a scene
@@ -196,8 +196,9 @@ __global__ void k_group_nbr(const int4* __restrict__ group_page, int64_t G, Page
 }
 
 // ------------------------------------------------------ binning by page ----
-// Groups up to which comparing all pairs (k_rank) is worth it.  A pass by page
-// and by radix sort, 2 particles per group: 5000 groups 0.122 ms by page, 7000
+// Groups up to which binning by page is worth it: k_rank compares all pairs (40 us
+// at 7500 groups) and k_number numbers the pages in one CTA (132 us).  A pass by
+// page and by radix sort, 2 particles per group: 5000 groups 0.122 ms by page, 7000
 // 0.214 and 0.231, 8000 0.258 and 0.226, 16000 0.545 and 0.267; 128 per group: 7000
 // 0.325 and 0.38, 8000 0.383 and 0.40, 16000 0.79 and 0.59.  In a substep, where the
 // radix way's 30 launches more also leave gaps, the two meet between 8400 and

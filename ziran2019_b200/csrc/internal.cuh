@@ -75,20 +75,15 @@ struct SolverScalars {
     int32_t kactive;           // 1 while the current linear solve iterates
     int32_t kit;               // Krylov iteration index of the current linear solve
     int32_t nit;               // Newton iteration index (= Newton loop bodies run)
-    int32_t krylov_bodies;     // Krylov loop bodies run (graph launch accounting)
-    uint32_t ticket;           // CTAs of the running kernel that finished (last_cta); 0 between kernels
     int32_t newton_iters;      // linear solves run
     int32_t krylov_iters;      // summed Krylov iterations
     int32_t hvp_count;
     int32_t converged;
     int32_t fp64_res;          // MIXED: 1 once the Newton residual is evaluated in FP64 (its FP32 form stalled)
-    int32_t skip_step;         // 1: this Newton iteration takes no step (the residual is re-evaluated first)
     int32_t kcount[64];        // Krylov iterations of each Newton iteration
     double res_initial, res_final;
     double rel_tol, local_tol;
     double rnorm;              // current preconditioned residual norm of the linear solve
-    // CG
-    double zTrk;
     // MINRES (Minres.h:16-24), double buffered by iteration parity
     double mr[2][12];
     // delta, epsilon, gamma, t and beta of the last MINRES iteration: its
@@ -269,14 +264,13 @@ int begin_edit(Ctx* ctx);  // download, then mark the device copy stale
 int run_explicit(Ctx* ctx, const zmpm_solver& s);      // symplectic substep up to G2P
 int launch_explicit_force(Ctx* ctx, double* out, bool mls); // out -= the explicit substep's forces (stress and scatter)
 int run_phase_field(Ctx* ctx, int32_t* iterations, double* residual); // FractureSimulation::solvePhaseFieldSystem after P2G
-int launch_phase_field_delete(Ctx* ctx);                               // FractureSimulation::deleteParticles before binning                  // V0 tau(F) (+ V0 tau(Fe)) into the stress buffer
+int launch_phase_field_delete(Ctx* ctx);                               // FractureSimulation::deleteParticles before binning
 int launch_update(Ctx* ctx, bool gated = true);       // G2P(vn+dv) -> stress -> force P2G
 int launch_adj_g2p(Ctx* ctx, double* vsbar);           // adjoint of G2P (adjoint.cu)
 int launch_adj_particle(Ctx* ctx, const double* lam);  // adjoint of the force term, P2G and E
 int run_adjoint_solve(Ctx* ctx, double tol, int max_iterations); // (M + dt^2 K) lambda = P dL/dv*
 int launch_residual(Ctx* ctx);                         // r = dt m g + dt f - m dv (projected), norm partials
 int launch_hvp(Ctx* ctx, const double* x, double* out, bool fp32); // out += dt^2 K x (no inertia)
-// FP32 product inside the MINRES loop of a MIXED context, on the FP32 copies x0 / x1 (even / odd iterations)
 int launch_damage(Ctx* ctx);                           // Rankine damage after P2G
 int run_admm(Ctx* ctx, const zmpm_solver& s);         // AdmmSimulation::admmStep
 // particle kernels of the ADMM substep (admm.cu)
@@ -290,7 +284,6 @@ int launch_admm_lastdv(Ctx* ctx);                      // last_dv = sum dv w / (
 int launch_force_scatter(Ctx* ctx, double* out);       // out -= sum_p stress_p grad w_ip (stress buffer)
 int finalize_multiply(Ctx* ctx, const double* x, double* q); // q = project(m x + q)
 int ensure_node_buffers(Ctx* ctx);
-int compute_node_indices(Ctx* ctx);                    // getNumNodes numbering (hooks)
 
 } // namespace zmpm
 

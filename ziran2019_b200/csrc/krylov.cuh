@@ -230,7 +230,6 @@ __device__ __forceinline__ void mr_store(SolverScalars* sc, const double* mst, i
     sc->rnorm = rnorm;
     sc->krylov_iters += 1;
     sc->hvp_count += 1;
-    sc->krylov_bodies += 1;
     if (nit < 64) sc->kcount[nit] += 1;
     sc->kit = k;
     if (!go) sc->kactive = 0;

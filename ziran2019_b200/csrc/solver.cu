@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_krylov_start(NodeGeom ng, Krylov
     const double rnorm = sqrt(dotv);
     const double rel = sc->rel_tol;
     const double lt = fmin(rel * rnorm, np.abs_tol);
-    const bool active = !(rnorm < lt) && np.kmax > 0 && !sc->skip_step;
+    const bool active = !(rnorm < lt) && np.kmax > 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->rnorm = rnorm;
         sc->local_tol = lt;
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_krylov_start(NodeGeom ng, Krylov
             mr[MR_BETA_KP1] = rnorm;
         }
         else
-            sc->mr[0][0] = dotv; // CG keeps zTrk double-buffered in mr[parity][0]
+            sc->mr[0][0] = dotv; // CG keeps z . r double-buffered in mr[parity][0]
     }
 }
 
@@ -736,7 +736,6 @@ __global__ void __launch_bounds__(FUSED_THREADS, HvpSmem<L, T, TX>::CTAS) k_cg_p
             sc->rnorm = rnorm;
             sc->krylov_iters += 1;
             sc->hvp_count += 1;
-            sc->krylov_bodies += 1;
             if (nit < 64) sc->kcount[nit] += 1;
             sc->kit = k;
             if (!go) sc->kactive = 0;
