@@ -66,3 +66,21 @@ def test_no_room_for_the_coefficients(cuda_lib, oracle, precision):
         for k in ("X", "V", "F"):
             assert np.abs(a[k] - b[k]).max() <= tol * np.abs(b[k]).max(), (n, k)
     assert free == 2 and n > 30
+
+
+@pytest.mark.parametrize("cells,ppc", [((9, 7, 11), 8), ((12, 12, 12), 1)])
+def test_mixed_substep_repeats(cuda_lib, cells, ppc):
+    """MIXED sums the FP32 coefficients in the order its atomics arrive: from one checkpoint the velocities repeat to
+    FP32's rounding and the Krylov counts to one iteration."""
+    s = make(None, block(cells, ppc, 4), "mixed", "auto", 6)
+    s.checkpointSave(0)
+    assert s.advanceOneTimeStep(2e-3) == abi.OK
+    s.checkpointSave(0)
+    v, counts = [], []
+    for _ in range(6):
+        s.checkpointLoad(0)
+        assert s.advanceOneTimeStep(2e-3) == abi.OK
+        v.append(s.getParticles()["V"])
+        counts.append(s.last_stats["krylov_iterations"])
+    assert max(counts) - min(counts) <= 1
+    assert max(np.linalg.norm(a - v[0]) for a in v) <= 2 * 2.0 ** -24 * np.linalg.norm(v[0])
